@@ -398,6 +398,41 @@ def test_device_dup_modes_match_reference(gpu_ctx, reflib, mode):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(1,), (127, 129), (128, 1, 256), (60, 70, 300)],
+                         ids=lambda s: "-".join(map(str, s)))
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_device_dup_modes_match_restatement(gpu_ctx, mode, sizes):
+    """The tiled pair tests at tile edges and with events sharing a tile
+    (seed counts around 128 per event), against the restatement on the
+    device's own exported tracks: bit-exact."""
+    from mkfit_b200 import synth
+    from mkfit_b200.finder import prepare_event_host
+    from mkfit_b200.seed_clean import cleaned_event
+    evs = []
+    for i, n in enumerate(sizes):
+        ev = synth.gen_cms_event(max(2 * n, 30), seed=71 + i, noise_frac=0.02)
+        sd = synth.with_duplicate_seeds(ev, frac=0.4, seed=71 + i)
+        keep = (np.arange(len(sd["chg"])) < n).astype(np.int32)
+        evs.append(cleaned_event(ev, sd, (keep, sd["nhits"], sd["hit_layer"], sd["hit_index"])))
+        assert evs[-1].n_seeds == n
+    frac, drth = (0.14, (0.001, 0.001, 0.001)) if mode == 1 else (0.24, (0.002, 0.004, 0.008))
+    fnd = _finder(gpu_ctx)
+    fnd.upload_batch(evs)
+    fnd.run()
+    N = sum(sizes)
+    keep = fnd.select(N, mode=mode, algorithm=4, frac_shared_hits=frac, drth_central=drth[0],
+                      drth_obarrel=drth[1], drth_forward=drth[2])
+    c = fnd.download_best(N)
+    exp = np.zeros(N, np.int32)
+    begin = 0
+    for e in evs:
+        tracks, idx = _sorted_exports(c, begin, prepare_event_host(e, fnd.cfg)["seed_order"])
+        exp[idx] = restate_dups(mode, tracks, algo=4, frac=frac, drth=drth)
+        begin += e.n_seeds
+    np.testing.assert_array_equal(keep, exp)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("it", [5, 7, 8, 9])
 def test_iteration_selection_matches_reference(gpu_ctx, reflib, it):
     """run_OneIteration's steps after the clone engine with the selection of
