@@ -14,8 +14,11 @@
 //      later seed (by index) of its event in the eta bins within reach (an
 //      overlap needs |d eta| < drmax), appending overlapping pairs;
 //   4. k_clean_resolve (block per event): the event's pairs sorted by
-//      (ts, tss) in shared memory, then one thread replays the reference's
-//      loop over them in that order (skip, drop, hit merge, layer sort).
+//      (ts, tss) in shared memory and split into connected components; one
+//      thread per component replays the reference's loop over its pairs in
+//      that order (skip, drop, hit merge, layer sort). A pair only reads
+//      and writes its own two seeds, so pairs of different components do
+//      not interact and the order within a component is the whole order.
 // Overlapping pairs are rare, so step 4 is short; the O(n^2) scan of the
 // reference becomes a scan over eta neighbours.
 #include "internal.h"
@@ -45,7 +48,7 @@ struct CleanParams {
 struct CleanDev {
   int n_events;
   const int* ev_begin;  // [n_events + 1]
-  const int* ev_of;     // [n] event of each seed
+  int* ev_of;           // [n] event of each seed
   int n;
   const float* par;     // [6][n]
   const int* chg;
@@ -59,16 +62,17 @@ struct CleanDev {
   int* ebin;            // [n]
   int* bin_count;       // [n_events][kEtaBins + 1]
   int* order;           // [n] seeds of each event by eta bin
-  int2* pairs;          // overlapping (ts, tss), global seed indices
-  int* pair_ev;         // event of each pair
-  int* n_pairs;
-  int pair_cap;
+  int2* pairs;          // [n_events][pair_stride] overlapping (ts, tss), global seed indices
+  int pair_stride;
+  int* ev_pairs;        // [n_events] pairs of each event
+  int* n_pairs;         // all pairs
+  int* comp;            // [n] component label: smallest seed of the component
   int max_hits;
   int* nh;              // [n]
   int* hl;              // [n][max_hits] hit layer
   int* hi;              // [n][max_hits] hit index
   int* keep;            // [n]
-  int* err;             // bit 0: pair pool overflow, bit 1: per-event pair overflow
+  int* err;             // bit 1: per-event pair overflow
 };
 
 __global__ void k_clean_features(CleanDev D, CleanParams P) {
@@ -78,6 +82,15 @@ __global__ void k_clean_features(CleanDev D, CleanParams P) {
   const float ipt = D.par[3 * D.n + i], phi = D.par[4 * D.n + i], theta = D.par[5 * D.n + i];
   const int q = D.chg[i];
   (void)z;
+  // The seed's event: the last one that begins at or before it (empty
+  // events share their begin with the next one).
+  int lo = 0, hi = D.n_events - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (D.ev_begin[mid] <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  D.ev_of[i] = lo;
   const float pt = fabsf(1.f / ipt);
   D.pt[i] = pt;
   const float eta = eta_of_theta(theta);
@@ -93,8 +106,20 @@ __global__ void k_clean_features(CleanDev D, CleanParams P) {
   const float f = (eta - kEtaLo) * (kEtaBins / (kEtaHi - kEtaLo));
   const int b = f >= 0.f ? min((int)f, kEtaBins - 1) : 0;
   D.ebin[i] = b;
-  atomicAdd(&D.bin_count[D.ev_of[i] * (kEtaBins + 1) + b], 1);
+  atomicAdd(&D.bin_count[lo * (kEtaBins + 1) + b], 1);
   D.keep[i] = 1;
+}
+
+// The output hit rows (max_hits wide, zero-filled) from the given ones
+// (in_hits wide): padded here, so the narrow rows cross the bus.
+__global__ void k_clean_rows(CleanDev D, const int* __restrict__ in_hl, const int* __restrict__ in_hi,
+                             int in_hits) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)D.n * D.max_hits) return;
+  const int i = (int)(t / D.max_hits), k = (int)(t % D.max_hits);
+  const bool on = k < D.nh[i];
+  D.hl[t] = on ? in_hl[(size_t)i * in_hits + k] : 0;
+  D.hi[t] = on ? in_hi[(size_t)i * in_hits + k] : 0;
 }
 
 // Exclusive scan of an event's histogram into bin starts, then the seeds
@@ -190,13 +215,8 @@ __global__ void __launch_bounds__(kCleanBlock) k_clean_pairs(CleanDev D, CleanPa
   for (int k = start[b0]; k < start[b1 + 1]; ++k) {
     const int tss = D.order[s0 + k];
     if (tss <= ts || !seeds_overlap(D, P, ts, tss)) continue;
-    const int at = atomicAdd(D.n_pairs, 1);
-    if (at >= D.pair_cap) {
-      atomicOr(D.err, 1);
-      continue;
-    }
-    D.pairs[at] = make_int2(ts, tss);
-    D.pair_ev[at] = e;
+    const int at = atomicAdd(D.ev_pairs + e, 1);
+    if (at < D.pair_stride) D.pairs[(size_t)e * D.pair_stride + at] = make_int2(ts, tss);
   }
 }
 
@@ -252,23 +272,27 @@ __device__ void sort_seed_hits(const CleanDev& D, int s) {
   }
 }
 
+// Latency bound: a component's replay is a chain of dependent reads of its
+// seeds' hit lists, so components run side by side, one thread each (one
+// thread for the whole event took 2003 us for 32 events of 3600 seeds and
+// about 700 pairs each, a third of the whole host-buffer call).
 __global__ void __launch_bounds__(kResolveBlock) k_clean_resolve(CleanDev D) {
   __shared__ long long s_key[kMaxEventPairs];
-  __shared__ int s_n;
+  __shared__ int s_comp[kMaxEventPairs];  // component of each sorted pair
   const int e = blockIdx.x, tid = threadIdx.x;
-  if (tid == 0) s_n = 0;
-  __syncthreads();
-  const int np = min(*D.n_pairs, D.pair_cap);
-  for (int p = tid; p < np; p += kResolveBlock) {
-    if (D.pair_ev[p] != e) continue;
-    const int at = atomicAdd(&s_n, 1);
-    if (at < kMaxEventPairs)
-      s_key[at] = ((long long)D.pairs[p].x << 32) | (unsigned)D.pairs[p].y;
-    else
-      atomicOr(D.err, 2);
+  const int found = D.ev_pairs[e];
+  if (tid == 0 && found) {
+    atomicAdd(D.n_pairs, found);
+    if (found > kMaxEventPairs) atomicOr(D.err, 2);
   }
-  __syncthreads();
-  const int n = min(s_n, kMaxEventPairs);
+  const int n = min(found, D.pair_stride);
+  for (int p = tid; p < n; p += kResolveBlock) {
+    const int2 pr = D.pairs[(size_t)e * D.pair_stride + p];
+    s_key[p] = ((long long)pr.x << 32) | (unsigned)pr.y;
+    // Every seed starts as its own component.
+    D.comp[pr.x] = pr.x;
+    D.comp[pr.y] = pr.y;
+  }
   int m = 1;
   while (m < n) m <<= 1;
   for (int i = n + tid; i < m; i += kResolveBlock) s_key[i] = LLONG_MAX;
@@ -290,28 +314,57 @@ __global__ void __launch_bounds__(kResolveBlock) k_clean_resolve(CleanDev D) {
       __syncthreads();
     }
   }
-  if (tid != 0) return;
-  // The reference's loops over the overlapping pairs, in its order.
-  int cur = -1, added = 0;
-  bool skip = false;
-  for (int p = 0; p < n; ++p) {
-    const int ts = (int)(s_key[p] >> 32), tss = (int)(s_key[p] & 0xffffffffLL);
-    if (ts != cur) {
-      cur = ts;
-      skip = !D.keep[ts];  // dropped by an earlier seed: the outer loop skips it
-      added = 0;
+  // Components: the smaller label of a pair spreads to its other seed, and
+  // to the seed that gave the larger label, until no label changes (each
+  // sweep that changes one lowers a label, so it ends; chains of duplicates
+  // are a few seeds long).
+  bool changed = n > 0;
+  while (__syncthreads_or(changed)) {
+    changed = false;
+    for (int p = tid; p < n; p += kResolveBlock) {
+      const int a = (int)(s_key[p] >> 32), b = (int)(s_key[p] & 0xffffffffLL);
+      const int la = atomicAdd(D.comp + a, 0), lb = atomicAdd(D.comp + b, 0);
+      if (la == lb) continue;
+      changed = true;
+      const int lo = min(la, lb);
+      atomicMin(D.comp + a, lo);
+      atomicMin(D.comp + b, lo);
+      atomicMin(D.comp + max(la, lb), lo);
     }
-    if (skip) continue;
-    int i1 = ts, i2 = tss;
-    if (D.d0[tss] > D.d0[ts]) {
-      D.keep[tss] = 0;
-    } else {
-      D.keep[ts] = 0;
-      i1 = tss;
-      i2 = ts;
+  }
+  for (int p = tid; p < n; p += kResolveBlock)
+    s_comp[p] = atomicAdd(D.comp + (int)(s_key[p] >> 32), 0);
+  __syncthreads();
+  // The component's smallest seed is the first of its pairs' ts (a pair
+  // holding it has it as ts, and the pairs are sorted by ts): the thread of
+  // the first pair of that ts replays the component.
+  for (int head = tid; head < n; head += kResolveBlock) {
+    const int root = (int)(s_key[head] >> 32);
+    if (s_comp[head] != root) continue;
+    if (head > 0 && (int)(s_key[head - 1] >> 32) == root) continue;
+    // The reference's loops over the overlapping pairs, in its order.
+    int cur = -1, added = 0;
+    bool skip = false;
+    for (int p = head; p < n; ++p) {
+      if (s_comp[p] != root) continue;
+      const int ts = (int)(s_key[p] >> 32), tss = (int)(s_key[p] & 0xffffffffLL);
+      if (ts != cur) {
+        cur = ts;
+        skip = !D.keep[ts];  // dropped by an earlier seed: the outer loop skips it
+        added = 0;
+      }
+      if (skip) continue;
+      int i1 = ts, i2 = tss;
+      if (D.d0[tss] > D.d0[ts]) {
+        D.keep[tss] = 0;
+      } else {
+        D.keep[ts] = 0;
+        i1 = tss;
+        i2 = ts;
+      }
+      added += merge_seed_hits(D, i1, i2);
+      if (added > 0) sort_seed_hits(D, i1);
     }
-    added += merge_seed_hits(D, i1, i2);
-    if (added > 0) sort_seed_hits(D, i1);
   }
 }
 
@@ -360,20 +413,20 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   MKFG_REQUIRE(drmax > 0.f && drmax < 1.f, "drmax out of range");
   P.reach = (int)std::ceil(drmax * (kEtaBins / (kEtaHi - kEtaLo))) + 1;
 
-  std::vector<int> ev_of(n);
-  for (int e = 0; e < n_events; ++e)
-    for (int i = event_seed_begin[e]; i < event_seed_begin[e + 1]; ++i) ev_of[i] = e;
-  std::vector<int> hl((size_t)n * max_hits, 0), hi((size_t)n * max_hits, 0);
-  for (int i = 0; i < n; ++i)
-    for (int k = 0; k < seed_nhits[i]; ++k) {
-      hl[(size_t)i * max_hits + k] = seed_hit_layer[(size_t)i * in_hits + k];
-      hi[(size_t)i * max_hits + k] = seed_hit_index[(size_t)i * in_hits + k];
-    }
-
+  // Pairs an event can have: what the resolve step holds, and never more
+  // than its seeds allow.
+  long long most = 1;
+  for (int e = 0; e < n_events; ++e) {
+    const long long m = event_seed_begin[e + 1] - event_seed_begin[e];
+    most = std::max(most, m * (m - 1) / 2);
+  }
+  const int pair_stride = (int)std::min<long long>(most, kMaxEventPairs);
   const int pair_cap = 8 * n + 1024;
   const size_t f_bytes = 4 * (size_t)n;
-  const size_t need = 6 * f_bytes * 4 + 4 * (size_t)n_events * (kEtaBins + 1) + 4 * (size_t)(n_events + 1) +
-                      12 * (size_t)pair_cap + 8 * (size_t)n * max_hits + 64 + 64 * 256;
+  const size_t row_bytes = 4 * (size_t)n * in_hits, out_bytes = 4 * (size_t)n * max_hits;
+  const size_t need = 6 * f_bytes * 4 + 4 * (size_t)n_events * (kEtaBins + 3) +
+                      8 * (size_t)n_events * pair_stride + 2 * row_bytes + 2 * out_bytes + 64 +
+                      64 * 256;
   if ((rc = ctx->scratch_misc.ensure(need))) return rc;
   char* base = ctx->scratch_misc.as<char>();
   size_t off = 0;
@@ -386,7 +439,7 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   D.n_events = n_events;
   D.n = n;
   D.max_hits = max_hits;
-  D.pair_cap = pair_cap;
+  D.pair_stride = pair_stride;
   float* par = (float*)take(6 * f_bytes);
   int* chg = (int*)take(f_bytes);
   D.par = par;
@@ -405,12 +458,15 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   D.ebin = (int*)take(f_bytes);
   D.bin_count = (int*)take(4 * (size_t)n_events * (kEtaBins + 1));
   D.order = (int*)take(f_bytes);
-  D.pairs = (int2*)take(8 * (size_t)pair_cap);
-  D.pair_ev = (int*)take(4 * (size_t)pair_cap);
+  D.pairs = (int2*)take(8 * (size_t)n_events * pair_stride);
+  D.comp = (int*)take(f_bytes);
   D.nh = (int*)take(f_bytes);
-  D.hl = (int*)take(4 * (size_t)n * max_hits);
-  D.hi = (int*)take(4 * (size_t)n * max_hits);
+  D.hl = (int*)take(out_bytes);
+  D.hi = (int*)take(out_bytes);
+  int* in_hl = (int*)take(row_bytes);
+  int* in_hi = (int*)take(row_bytes);
   D.keep = (int*)take(f_bytes);
+  D.ev_pairs = (int*)take(4 * (size_t)n_events);
   int* flags = (int*)take(64);
   D.n_pairs = flags;
   D.err = flags + 1;
@@ -420,14 +476,16 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   MKFG_CUDA_TRY(cudaMemcpyAsync(par, seed_par, 6 * f_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(chg, seed_chg, f_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(evb, event_seed_begin, 4 * (size_t)(n_events + 1), cudaMemcpyHostToDevice, st));
-  MKFG_CUDA_TRY(cudaMemcpyAsync(evo, ev_of.data(), f_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(D.nh, seed_nhits, f_bytes, cudaMemcpyHostToDevice, st));
-  MKFG_CUDA_TRY(cudaMemcpyAsync(D.hl, hl.data(), 4 * hl.size(), cudaMemcpyHostToDevice, st));
-  MKFG_CUDA_TRY(cudaMemcpyAsync(D.hi, hi.data(), 4 * hi.size(), cudaMemcpyHostToDevice, st));
+  MKFG_CUDA_TRY(cudaMemcpyAsync(in_hl, seed_hit_layer, row_bytes, cudaMemcpyHostToDevice, st));
+  MKFG_CUDA_TRY(cudaMemcpyAsync(in_hi, seed_hit_index, row_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemsetAsync(D.bin_count, 0, 4 * (size_t)n_events * (kEtaBins + 1), st));
   MKFG_CUDA_TRY(cudaMemsetAsync(flags, 0, 64, st));
+  MKFG_CUDA_TRY(cudaMemsetAsync(D.ev_pairs, 0, 4 * (size_t)n_events, st));
   const int grid = (n + kCleanBlock - 1) / kCleanBlock;
   k_clean_features<<<grid, kCleanBlock, 0, st>>>(D, P);
+  const long long cells = (long long)n * max_hits;
+  k_clean_rows<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(D, in_hl, in_hi, in_hits);
   k_clean_bins<<<n_events, kCleanBlock, 0, st>>>(D);
   k_clean_pairs<<<grid, kCleanBlock, 0, st>>>(D, P);
   k_clean_resolve<<<n_events, kResolveBlock, 0, st>>>(D);
@@ -435,11 +493,11 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   int h_flags[2] = {0, 0};
   MKFG_CUDA_TRY(cudaMemcpyAsync(keep, D.keep, f_bytes, cudaMemcpyDeviceToHost, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(out_nhits, D.nh, f_bytes, cudaMemcpyDeviceToHost, st));
-  MKFG_CUDA_TRY(cudaMemcpyAsync(out_hit_layer, D.hl, 4 * hl.size(), cudaMemcpyDeviceToHost, st));
-  MKFG_CUDA_TRY(cudaMemcpyAsync(out_hit_index, D.hi, 4 * hi.size(), cudaMemcpyDeviceToHost, st));
+  MKFG_CUDA_TRY(cudaMemcpyAsync(out_hit_layer, D.hl, out_bytes, cudaMemcpyDeviceToHost, st));
+  MKFG_CUDA_TRY(cudaMemcpyAsync(out_hit_index, D.hi, out_bytes, cudaMemcpyDeviceToHost, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(h_flags, flags, 8, cudaMemcpyDeviceToHost, st));
   MKFG_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h_flags[1] & 1) return set_error(MKFG_ERR_OVERFLOW, "seed cleaning: more than %d overlapping pairs", pair_cap);
+  if (h_flags[0] > pair_cap) return set_error(MKFG_ERR_OVERFLOW, "seed cleaning: more than %d overlapping pairs", pair_cap);
   if (h_flags[1] & 2)
     return set_error(MKFG_ERR_OVERFLOW, "seed cleaning: more than %d overlapping pairs in one event", kMaxEventPairs);
   return MKFG_OK;

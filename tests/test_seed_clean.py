@@ -143,3 +143,38 @@ def test_device_large_batch_properties(gpu_ctx, reflib):
         hits = list(zip(hi[i, :nh[i]], hl[i, :nh[i]]))
         assert len(set(hits)) == len(hits)
         assert list(hl[i, :nh[i]]) == sorted(hl[i, :nh[i]])
+
+
+@pytest.mark.gpu
+def test_device_components_match_restatement(gpu_ctx):
+    """Connected components of duplicates, replayed side by side: a batch
+    with an empty event, one of a single seed, ordinary near-duplicates and
+    a long chain (15 exact copies interleaved with other seeds: one
+    component, whose merges reach the 15-hit cap), against the restatement
+    per event."""
+    from mkfit_b200.seed_clean import clean_seeds
+    first = lambda k, v, n: v[:, :n] if k in ("par", "err") else v[:n]  # noqa: E731
+    chain = seeds_of(40, 7, frac=0.3)
+    n = len(chain["chg"])
+    chain = {k: np.concatenate([v] + [first(k, v, 1)] * 14, axis=1 if k in ("par", "err") else 0)
+             for k, v in chain.items()}
+    chain["hit_index"][n:, 2] = 1000 + np.arange(14)
+    order = np.random.default_rng(3).permutation(n + 14)
+    chain = {k: v[:, order] if k in ("par", "err") else v[order] for k, v in chain.items()}
+    evs = [seeds_of(130, 41), first_event(seeds_of(5, 42, frac=0.0), 0),
+           first_event(seeds_of(5, 42, frac=0.0), 1), chain, seeds_of(60, 43)]
+    begin = np.cumsum([0] + [len(e["chg"]) for e in evs]).astype(np.int32)
+    cat = lambda k, ax: np.concatenate([e[k] for e in evs], axis=ax)  # noqa: E731
+    out = clean_seeds(gpu_ctx, begin, cat("par", 1), cat("chg", 0), cat("nhits", 0),
+                      cat("hit_layer", 0), cat("hit_index", 0))
+    for e, sd in enumerate(evs):
+        a, b = begin[e], begin[e + 1]
+        if a == b:
+            continue
+        exp = restate_clean_seeds(sd, PARAMS)
+        assert device_mismatches(tuple(x[a:b] for x in out), exp, sd) <= 1
+    assert out[1].max() == 15
+
+
+def first_event(sd, n):
+    return {k: (v[:, :n] if k in ("par", "err") else v[:n]) for k, v in sd.items()}
