@@ -55,10 +55,10 @@ constexpr int kBlock = 256;
 #ifndef MKFG_ACT_MIN_BLOCKS
 #define MKFG_ACT_MIN_BLOCKS 8
 #endif
-// The same for the clone kernel (one warp per seed, latency bound: the
-// full 64 warps per SM pay for the few registers spilled to L1).
+// The clone kernel, bound by dependent loads: 64 registers at 4 blocks
+// (5.26 ms per 64-event step; 5 blocks 5.79, 6 blocks 7.54: spills).
 #ifndef MKFG_CLONE_MIN_BLOCKS
-#define MKFG_CLONE_MIN_BLOCKS 8
+#define MKFG_CLONE_MIN_BLOCKS 4
 #endif
 
 
@@ -421,71 +421,60 @@ __global__ void __launch_bounds__(kBlock, MKFG_CHI2_MIN_BLOCKS) k_chi2(EventDev 
 
 //------------------------------------------------------------------------------
 // Kernel 3: per-seed candidate cloning (CandCloner::ProcessSeedRange,
-// mkFit/CandCloner.cc:36-189). One warp per seed.
+// mkFit/CandCloner.cc:36-189), 8 lanes per seed: one per candidate, then
+// one per new candidate, so every access to the 8 slots of a seed covers
+// one 32-byte sector. The state of a candidate that takes an update is left
+// to the update kernel, which reads it from the parent. The kernel is bound
+// by its chain of dependent loads (list, masks, records, parent), so the
+// fewer instructions a seed takes the more of them are in flight: a warp
+// per seed issued 970 instructions for work that keeps 8 lanes busy, a
+// thread per seed left 10 warps on an SM (260 us in the busiest step of the
+// 64-event batch). 64-event batch, 42 steps: clone 5.26 against 7.52 ms a
+// warp per seed, with the update at 2.33 against 1.93 (it now gathers the
+// parents' states); 3.9 TB/s of DRAM traffic, 270 instructions per seed.
 //------------------------------------------------------------------------------
 // kCount: also count the records present and the new candidates (work
-// counters 4 and 5). The eager launch sequence counts; the graph form, whose
-// kernel sits at its register cap, does not.
+// counters 4 and 5), for the eager launch sequence.
+constexpr int kClonePerBlock = kBlock / kSlots;
+
 template <bool kCount>
 __global__ void __launch_bounds__(kBlock, MKFG_CLONE_MIN_BLOCKS) k_clone(EventDev E, const FindConfigDev* __restrict__ Cp,
                                                   int step) {
   const FindConfigDev& C = *Cp;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __shared__ HitMatchPair s_hm[kBlock / 32][kSlots];
-  __shared__ CloneScratch s_scratch[kBlock / 32];
+  const int lane = threadIdx.x & 31, ls = threadIdx.x / kSlots, c = threadIdx.x % kSlots;
+  __shared__ CloneScratch s_scratch[kClonePerBlock];
   __shared__ BlockAppend sh;
-  __shared__ int s_work[2];  // records present, new candidates (this block)
-  HitMatchPair* hm = s_hm[warp];
   int* cnt = E.step_count + step * kCntN;
   const int n_find = cnt[kCntFind];
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&E.work[step * kWorkN + 3], n_find);
-  if (kCount) {
-    if (threadIdx.x < 2) s_work[threadIdx.x] = 0;
-    __syncthreads();
-  }
-  // Block-uniform loop (the update-list append synchronises the block):
-  // warp `warp` of the block takes seed base + warp of each round.
-  for (int base = blockIdx.x * (kBlock / 32); base < n_find; base += gridDim.x * (kBlock / 32)) {
-    const int w = base + warp;
-    int u = 0, g = 0, slot = 0, upd_info = 0;
-    bool barrel = true;
-    if (w < n_find) {
-      // A seed finding at this step (listed by the activation kernel).
-      const int s = E.find_list[w];
-      const int info = E.find_info[w];
-      const int cur = info & 1, ncand = (info >> 1) & 15, layer = info >> 5;
-      const size_t rb = (size_t)s * kRecPerSeed;
-      const int hit0 = E.layer_begin[E.seed_event[s] * E.lb_stride + layer];
-      const SeedRecords R{E.rec + rb, E.rmask + s * kSlots, E.wsr + s * kSlots,
-                          E.extra_last + s * kSlots, nullptr};
-      int upd = 0, n_rec = 0;
-      const int n = clone_seed(E, C, s, layer, kFinding, ncand, cur, R, hm, s_scratch[warp], upd,
-                               lane, kCount ? &n_rec : nullptr);
-      if (n >= 0 && lane == 0) {
-        E.n_cands[s] = n;
-        E.cur[s] = cur ^ 1;
-      }
-      if (kCount && lane == 0) {
-        atomicAdd(s_work, n_rec);
-        atomicAdd(s_work + 1, max(n, 0));
-      }
-      // The new candidates that take a Kalman update, with the global index
-      // of the hit to update with (on this step's layer).
-      slot = s * kSlots + lane;
-      u = lane < n ? upd : 0;
-      g = u ? hit0 + (u - 1) : 0;
-      barrel = C.layer[layer].is_barrel;
-      // The new candidates sit in the other buffer.
-      upd_info = find_info_pack(cur ^ 1, 0, layer);
+  // Block-uniform loop (the update-list append synchronises the block).
+  for (int base = blockIdx.x * kClonePerBlock; base < n_find; base += gridDim.x * kClonePerBlock) {
+    const bool on = base + ls < n_find;
+    // A seed finding at this step (listed by the activation kernel).
+    const int s = on ? E.find_list[base + ls] : 0;
+    const int info = on ? E.find_info[base + ls] : 0;
+    const int cur = info & 1, ncand = (info >> 1) & 15, layer = info >> 5;
+    const SeedRecords R{E.rec + (size_t)s * kRecPerSeed, E.rmask + s * kSlots, E.wsr + s * kSlots,
+                        E.extra_last + s * kSlots};
+    const CloneList l = clone_rank(E, C, on, s, layer, ncand, cur, R, s_scratch[ls], lane);
+    if (on && c == 0) {
+      E.n_cands[s] = l.n;
+      E.cur[s] = cur ^ 1;
     }
-    append_two_ended_block(u != 0, barrel, slot, E.upd_list, E.list_cap, cnt + kCntUpdBarrel, sh, g,
-                           E.upd_hit, upd_info, E.upd_info);
-    __syncwarp();  // hm and scratch are reused by the next seed of this warp
-  }
-  if (kCount) {
-    __syncthreads();
-    if (threadIdx.x < 2 && s_work[threadIdx.x])
-      atomicAdd(&E.work[step * kWorkN + 4 + threadIdx.x], s_work[threadIdx.x]);
+    if (kCount && on && c == 0) {
+      atomicAdd(&E.work[step * kWorkN + 4], l.n_records);
+      atomicAdd(&E.work[step * kWorkN + 5], l.n);
+    }
+    int upd = 0;
+    if (on && c < l.n) upd = clone_write(E, s, layer, cur, R, l, c, false);
+    // The new candidates that take a Kalman update, with the global index
+    // of the hit to update with (on this step's layer) and where the
+    // parent's state is.
+    const bool barrel = C.layer[layer].is_barrel;
+    const int g = upd ? E.layer_begin[E.seed_event[s] * E.lb_stride + layer] + upd - 1 : 0;
+    append_two_ended_block(upd != 0, barrel, s * kSlots + c, E.upd_list, E.list_cap,
+                           cnt + kCntUpdBarrel, sh, g, E.upd_hit,
+                           find_info_pack(cur, l.parent, layer), E.upd_info);
   }
 }
 
@@ -503,7 +492,9 @@ __global__ void __launch_bounds__(kBlock, MKFG_UPD_MIN_BLOCKS) k_update(EventDev
     const int slot = E.upd_list[at];
     const int info = E.upd_info[at];
     const LayerDev& L = C.layer[info >> 5];
-    update_cand_at(E, C, L, E.upd_hit[at], E.cand[info & 1], slot);
+    const int cur = info & 1, parent = (info >> 1) & 15;
+    update_cand_at(E, C, L, E.upd_hit[at], E.cand[cur], (slot & ~(kSlots - 1)) + parent,
+                   E.cand[cur ^ 1], slot);
   }
 }
 
@@ -517,7 +508,6 @@ __global__ void k_reset(EventDev E, int n_work) {
   if (t == 0) E.err_flags[0] = 0;
   const int s = t / kSlots, c = t % kSlots;
   if (s >= E.n_seeds) return;
-  E.upd[t] = 0;
   if (c == 0) {
     copy_slot(E.init, s, E.cand[0], t);
     // A seed the upload's post-cleaning dropped (nfound < 0) has no
@@ -1121,25 +1111,26 @@ __global__ void k_update_last_hit(EventDev E, const FindConfigDev* __restrict__ 
 
 //------------------------------------------------------------------------------
 // CandCloner::ProcessSeedRange as a plain worker call (mkFit/CandCloner.cc:
-// 36-189): the clone step of the graph form (clone_seed) run on
-// caller-given candidates and records held in a private EventDev. One warp
-// per seed.
+// 36-189): the clone step of the graph form run on caller-given candidates
+// and records held in a private EventDev. 8 threads per seed.
 //------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock) k_clone_worker(EventDev W, const FindConfigDev* __restrict__ Cp,
                                                          int layer, int* __restrict__ n_new,
                                                          int* __restrict__ parent) {
   const FindConfigDev& C = *Cp;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __shared__ HitMatchPair s_hm[kBlock / 32][kSlots];
-  __shared__ CloneScratch s_scratch[kBlock / 32];
-  const int s = blockIdx.x * (kBlock / 32) + warp;
-  if (s >= W.n_seeds) return;
+  __shared__ CloneScratch s_scratch[kClonePerBlock];
+  const int ls = threadIdx.x / kSlots, c = threadIdx.x % kSlots;
+  const bool on = blockIdx.x * kClonePerBlock + ls < W.n_seeds;
+  const int s = on ? blockIdx.x * kClonePerBlock + ls : 0;
   const SeedRecords R{W.rec + (size_t)s * kRecPerSeed, W.rmask + s * kSlots, W.wsr + s * kSlots,
-                      W.extra_last + s * kSlots, W.upd + s * kSlots};
-  int upd = 0;
-  const int n = clone_seed(W, C, s, layer, kFinding, W.n_cands[s], 0, R, s_hm[warp], s_scratch[warp],
-                           upd, lane, nullptr, parent + s * kSlots);
-  if (lane == 0) n_new[s] = n;
+                      W.extra_last + s * kSlots};
+  const CloneList l = clone_rank(W, C, on, s, layer, on ? W.n_cands[s] : 0, 0, R, s_scratch[ls],
+                                 threadIdx.x & 31);
+  if (!on) return;
+  if (c == 0) n_new[s] = l.n;
+  if (c >= l.n) return;
+  W.upd[s * kSlots + c] = clone_write(W, s, layer, 0, R, l, c, true);
+  parent[s * kSlots + c] = l.parent;
 }
 
 __global__ void k_select_out(EventDev E, const SelectArgs A, const int* __restrict__ dup,
@@ -1907,7 +1898,7 @@ static int upload_batch(mkfg_context* ctx, Finder* f, const mkfg_event* evs, int
     f->ev.xhit = carve<int>(p, (size_t)kMaxXHits * SC);
     f->ev.wsr = carve<int>(p, SC);
     f->ev.extra_last = carve<int>(p, SC);
-    f->ev.upd = carve<int>(p, SC);
+    f->ev.upd = nullptr;
     f->ev.pairs = carve<int>(p, (size_t)SC * kMaxXHits);
     f->ev.pair_cap = SC * kMaxXHits;
     f->ev.pair_count = carve<int>(p, max_steps + 2);
@@ -2007,7 +1998,6 @@ static int upload_batch(mkfg_context* ctx, Finder* f, const mkfg_event* evs, int
   }
   if (S > 0) k_seed_nodes<<<(S + 127) / 128, 128, 0, st>>>(f->ev, f->seeds.as<int>());
   MKFG_CUDA_TRY(cudaGetLastError());
-  MKFG_CUDA_TRY(cudaMemsetAsync(f->ev.upd, 0, 4 * (size_t)SC, st));
   MKFG_CUDA_TRY(cudaMemsetAsync(f->ev.err_flags, 0, 64, st));
   // The pinned staging is reused by the next upload: wait for the copies.
   MKFG_CUDA_TRY(cudaStreamSynchronize(st));
@@ -2076,7 +2066,7 @@ static StepGrids step_grids(Finder* f) {
   g.activate = grid_c;
   g.propagate = std::min(grid_c, f->grid_mult[0] * f->resident[0]);
   g.chi2 = std::min((S * kSlots * 4 + kBlock - 1) / kBlock, f->grid_mult[1] * f->resident[1]);
-  g.clone = std::min((S * 32 + kBlock - 1) / kBlock, f->grid_mult[2] * f->resident[2]);
+  g.clone = std::min((S + kClonePerBlock - 1) / kClonePerBlock, f->grid_mult[2] * f->resident[2]);
   g.update = std::min(grid_c, f->grid_mult[3] * f->resident[3]);
   return g;
 }
@@ -3128,7 +3118,7 @@ extern "C" int mkfg_find_clone_seeds(mkfg_context* ctx, int32_t layer, const mkf
   MKFG_CUDA_TRY(cudaMemsetAsync(W.err_flags, 0, 4, st));
   MKFG_CUDA_TRY(cudaMemsetAsync(W.upd, 0, 4 * SC, st));
   MKFG_CUDA_TRY(cudaMemsetAsync(d_parent, 0xff, 4 * SC, st));
-  const int blocks = (S + kBlock / 32 - 1) / (kBlock / 32);
+  const int blocks = (S + kClonePerBlock - 1) / kClonePerBlock;
   k_clone_worker<<<blocks, kBlock, 0, st>>>(W, f->d_cfg, layer, d_new, d_parent);
   MKFG_CUDA_TRY(cudaGetLastError());
   // Read back.

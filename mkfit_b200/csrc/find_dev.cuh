@@ -139,7 +139,7 @@ struct EventDev {
   int* xhit;       // [kMaxXHits][S*kSlots] hit index within layer
   int* wsr;        // WSR code | extra kind << 8
   int* extra_last; // arena node of the held-back copy (kind 2)
-  int* upd;        // needs UpdateWithLastHit (per slot of the new buffer)
+  int* upd;        // update code per slot of the new buffer (clone worker call only)
   // Records (IdxChi2List) per seed: kRecPerSeed slots, kRecPerCand per
   // candidate (its hits in bin-scan order, then the hole record); a slot
   // holds a record when its bit of the candidate's mask is set.
@@ -162,9 +162,9 @@ struct EventDev {
   // (find_info_pack), so the clone kernel starts its loads from one read.
   int* find_list;
   int* find_info;
-  // Beside the update list: the candidate's buffer and layer
-  // (find_info_pack without the count), so the update starts its loads
-  // from its list entry.
+  // Beside the update list: the buffer and slot of the candidate's parent
+  // and the layer (find_info_pack with the slot in the count's place), so
+  // the update starts its loads from its list entry.
   int* upd_info;
   int* step_count; // [max_steps + 2][kCntN]
   int* err_flags;

@@ -1,10 +1,10 @@
 // Fused clone-engine finding: one thread block carries a chunk of W
 // consecutive seeds through every layer-plan step and the final merge in a
-// single launch. Per step the block runs the same four phases as the plain
-// form's four kernels (prep, chi2, clone, update), separated by block
+// single launch. Per step the block runs the same phases as the plain
+// form's kernels (prep, chi2, clone, update), separated by block
 // barriers, but the step scratch -- states propagated to the layer, selected
-// hit lists, the (candidate, hit) pair list, the IdxChi2List records, the
-// overlap pairs and the update flags -- lives in shared memory and never
+// hit lists, the (candidate, hit) pair list, and the IdxChi2List records
+// -- lives in shared memory and never
 // goes to DRAM. Candidate buffers, seed scalars and the hit-on-track arena
 // stay in global memory (each seed's data is touched by one block only, so
 // they stay in L1/L2 between phases).
@@ -26,12 +26,10 @@ struct FusedShared {
   int xhit[kMaxXHits * T];
   int wsr[T];
   int extra_last[T];
-  int upd[T];
   Record rec[W * kRecPerSeed];
   uint32_t rmask[T];
   unsigned short pairs[T * kMaxXHits];
-  HitMatchPair hm[T / 32][kSlots];
-  CloneScratch scratch[T / 32];
+  CloneScratch scratch[W];
   int n_pairs;
 };
 
@@ -43,7 +41,7 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
   extern __shared__ __align__(16) unsigned char fused_smem[];
   FusedShared<W>& S = *reinterpret_cast<FusedShared<W>*>(fused_smem);
   const FindConfigDev& C = *Cp;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int s0 = blockIdx.x * W;
   const int ls = tid / kSlots, c = tid % kSlots;  // local seed, candidate slot
   const int s = s0 + ls;
@@ -56,7 +54,6 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
   const int* lb = E.layer_begin + ev * E.lb_stride;
   const int n_local = min(W, E.n_seeds - s0);
 
-  S.upd[tid] = 0;
   if (tid == 0) S.n_pairs = 0;
   __syncthreads();
 
@@ -139,33 +136,27 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
 
     //-------------------------------------------------------------- clone
     if (tid == 0) S.n_pairs = 0;
-    for (int wl = warp; wl < n_local; wl += T / 32) {
-      const int ws = s0 + wl;
-      const int wlayer = plan_layer(C, E.region[ws], step);
-      if (wlayer < 0) continue;
-      const int wstate = E.state[ws];
-      if (wstate != kFinding) continue;
-      const int cur = E.cur[ws];
-      if (lane == 0) atomicAdd(&E.work[step * kWorkN + 3], 1);
-      const int rb = wl * kRecPerSeed;
-      const SeedRecords R{S.rec + rb, S.rmask + wl * kSlots, S.wsr + wl * kSlots,
-                          S.extra_last + wl * kSlots, S.upd + wl * kSlots};
-      int upd = 0;
-      const int n = clone_seed(E, C, ws, wlayer, wstate, E.n_cands[ws], cur, R, S.hm[warp],
-                               S.scratch[warp], upd, lane);
-      if (n >= 0 && lane == 0) {
-        E.n_cands[ws] = n;
-        E.cur[ws] = cur ^ 1;
+    // The 8 threads of a seed rank its records, then each writes a new
+    // candidate and updates it with the hit it took.
+    {
+      const bool on = in_range && layer >= 0 && state == kFinding && act != 0;
+      const SeedRecords R{S.rec + ls * kRecPerSeed, S.rmask + ls * kSlots, S.wsr + ls * kSlots,
+                          S.extra_last + ls * kSlots};
+      const CloneList l = clone_rank(E, C, on, on ? s : 0, layer, ncand, buf, R, S.scratch[ls], lane);
+      if (on && c == 0) {
+        atomicAdd(&E.work[step * kWorkN + 3], 1);
+        E.n_cands[s] = l.n;
+        E.cur[s] = buf ^ 1;
       }
-      __syncwarp();
-    }
-    __syncthreads();
-
-    //-------------------------------------------------------------- update
-    if (in_range && layer >= 0 && c < E.n_cands[s] && S.upd[tid]) {
-      S.upd[tid] = 0;
-      atomicAdd(&E.work[step * kWorkN + 1], 1);
-      update_cand(E, C, s, lb, E.cand[E.cur[s]], slot);
+      if (on && c < l.n) {
+        const int upd = clone_write(E, s, layer, buf, R, l, c, false);
+        //-------------------------------------------------------------- update
+        if (upd) {
+          atomicAdd(&E.work[step * kWorkN + 1], 1);
+          update_cand_at(E, C, C.layer[layer], lb[layer] + upd - 1, E.cand[buf],
+                         s * kSlots + l.parent, E.cand[buf ^ 1], slot);
+        }
+      }
     }
     // A seed can still change if it is dormant (it may wake up) or finding
     // with layers left in its plan.

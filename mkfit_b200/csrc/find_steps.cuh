@@ -273,15 +273,6 @@ namespace mkfg {
 // Shared step implementations (plain kernels and the fused persistent kernel)
 //------------------------------------------------------------------------------
 
-struct NewCand {
-  int parent;    // candidate slot (0..7) the new candidate copies
-  int hit;       // added hit index (or hole code)
-  float chi2hit;
-  int ov;        // overlap: match index 0/1 in the parent's pair, or -1
-  float score;
-  int is_extra;  // 1: held-back copy (extra), 2: extra with a stop (-2) node
-};
-
 // Every value is loaded before the first store: the compiler cannot tell
 // the two buffers apart, and interleaved loads and stores would wait for
 // one another (37 memory round trips instead of one).
@@ -529,30 +520,19 @@ __device__ __forceinline__ void update_state(const EventDev& E, const FindConfig
   }
 }
 
-// UpdateWithLastHit + CopyOutParErr for one candidate slot of buffer B
-// (MkFinder.cc:1291-1335), given the hit's global index g and its layer.
+// UpdateWithLastHit + CopyOutParErr for the new candidate in slot `slot` of
+// buffer N (MkFinder.cc:1291-1335): the state of its parent (slot `src` of
+// buffer B, which the clone step leaves where it is) updated with the hit
+// of global index g on layer L.
 __device__ __forceinline__ void update_cand_at(const EventDev& E, const FindConfigDev& C,
-                                               const LayerDev& L, int g, const CandSoA& B,
-                                               int slot) {
+                                               const LayerDev& L, int g, const CandSoA& B, int src,
+                                               const CandSoA& N, int slot) {
   float par[6], err[21];
-  load_state(B, slot, par, err);
-  int chg = B.chg[slot];
+  load_state(B, src, par, err);
+  int chg = B.chg[src];
   update_state(E, C, L, g, par, err, chg);
-  store_state(B, slot, par, err);
-  B.chg[slot] = chg;
-}
-
-// UpdateWithLastHit with the hit found from the candidate's last node.
-// Returns false if the last node is not a hit.
-__device__ __forceinline__ bool update_cand(const EventDev& E, const FindConfigDev& C, int s,
-                                            const int* lb, const CandSoA& B, int slot) {
-  const int hv = node_hot_of(E, s, B.last[slot]);
-  const int hl = hot_layer(hv);
-  // After an arena overflow (reported through err_flags) the last node may
-  // not be a hit: skip rather than read outside the hit arrays.
-  if (hot_index(hv) < 0 || hl < 0 || hl >= C.n_layers) return false;
-  update_cand_at(E, C, C.layer[hl], lb[hl] + hot_index(hv), B, slot);
-  return true;
+  store_state(N, slot, par, err);
+  N.chg[slot] = chg;
 }
 
 // Records and per-candidate step results of one seed, wherever they live
@@ -562,62 +542,24 @@ struct SeedRecords {
   const uint32_t* mask_;   // per candidate: bit h set = record h present
   const int* wsr_;         // WSR code | extra kind << 8, per candidate
   const int* extra_last_;  // stop node of a kind-2 extra, per candidate
-  int* upd_;               // per new candidate: 1 + index in its layer of the hit
-                           // to update with (the last one added), 0 = none;
-                           // null: returned only
   __device__ Record rec(int idx) const { return rec_[idx]; }
   __device__ uint32_t mask(int c) const { return mask_[c]; }
   __device__ int extra_kind(int c) const { return wsr_[c] >> 8; }
   __device__ int extra_last(int c) const { return extra_last_[c]; }
-  __device__ void set_upd(int i, int v) const {
-    if (upd_) upd_[i] = v;
-  }
 };
 
 // Total order of record scores as integers: the float order, with -0 taken
-// as +0 and NaN below every number (NaN records go last, in record order).
+// as +0 and NaN below every number (NaN records go last, in record order)
+// but above kNoKey, the key of an empty place.
+constexpr int kNoKey = INT_MIN;
 __device__ __forceinline__ int score_key(float score) {
   const float z = __fadd_rn(score, 0.f);
   const int k = __float_as_int(z);
-  return z != z ? INT_MIN : (k >= 0 ? k : k ^ 0x7fffffff);
+  return z != z ? kNoKey + 1 : (k >= 0 ? k : k ^ 0x7fffffff);
 }
-
-// Copy of the parameters and covariance of new candidates i < n (parent
-// slot parent_i, lane i of `parent`) from buffer B to buffer N, in two
-// halves so a caller can issue the loads early: load_par_err into seven
-// registers per lane, store_par_err from them. Lane t moves element
-// t / 8 + 4 k of candidate t % 8: each access of the warp covers four whole
-// 32-byte sectors (a seed's 8 slots are contiguous).
-__device__ __forceinline__ void load_par_err(const CandSoA& B, int s, int n, int parent, int lane,
-                                             float (&v)[7]) {
-  const int c = lane & 7;
-  const int pc = __shfl_sync(0xffffffffu, parent, c);
-  const int src = s * kSlots + pc;
-#pragma unroll
-  for (int k = 0; k < 7; ++k) {
-    const int e = (lane >> 3) + 4 * k;
-    v[k] = 0.f;
-    if (c < n && e < 27) v[k] = (e < 6 ? B.par + e * B.cap : B.err + (e - 6) * B.cap)[src];
-  }
-}
-__device__ __forceinline__ void store_par_err(const CandSoA& N, int s, int n, int lane,
-                                              const float (&v)[7]) {
-  const int c = lane & 7;
-  if (c >= n) return;
-  const int dst = s * kSlots + c;
-#pragma unroll
-  for (int k = 0; k < 7; ++k) {
-    const int e = (lane >> 3) + 4 * k;
-    float* to = e < 6 ? N.par + e * N.cap : N.err + (e - 6) * N.cap;
-    if (e < 27) to[dst] = v[k];
-  }
-}
-// Both halves at once (all loads before the first store).
-__device__ __forceinline__ void copy_par_err(const CandSoA& B, const CandSoA& N, int s, int n,
-                                             int parent, int lane) {
-  float v[7];
-  load_par_err(B, s, n, parent, lane, v);
-  store_par_err(N, s, n, lane, v);
+// The score a key stands for (+0 for -0, a NaN for any NaN).
+__device__ __forceinline__ float key_score(int key) {
+  return __int_as_float(key >= 0 ? key : key ^ 0x7fffffff);
 }
 
 // Writes a hit-on-track node at arena position pos of seed s (allocated by
@@ -635,336 +577,276 @@ __device__ __forceinline__ int arena_put(const EventDev& E, int s, int pos, int 
   return pos;
 }
 
-// Shared-memory scratch of one warp's clone step: the ranked records with
-// their fields, and the counters of the seed's candidates.
-struct CloneScratch {
-  int rec[32];
-  int hit[32];
-  float score[32];
-  float chi2[32];
-  int module[32];
-  // Per candidate: chg, chi2 bits, last, nfound, nmiss, nover, ninside,
-  // ntail, score bits, 1/pT bits, extra kind.
-  int cand[11][kSlots];
+// A seed's new candidates as the ranking leaves them, in the registers of
+// the 8 lanes that work on the seed: lane i holds new candidate i < n.
+struct CloneList {
+  int n;          // new candidates
+  int n_records;  // records present
+  int rec;        // record taken (index in the seed's records)
+  int parent;     // parent's slot
+  int kind;       // held-back copy: 1 plain, 2 with a stop node; 0 a record's candidate
+  int ov;         // parent's record of the overlap hit, or -1
+  int node;       // arena position of the candidate's first node
+  bool upd;       // takes an update
 };
 
-// CandCloner::ProcessSeedRange for one seed (mkFit/CandCloner.cc:36-189),
-// executed by one warp. Returns the new candidate count, or -1 when the
-// seed's candidates are unchanged; upd_out: lane i's new candidate's
-// update code (SeedRecords::upd_); n_records_out (optional): the records
-// present; parent_out (optional, kSlots entries): each new candidate's
-// parent slot. The warp owns the seed's arena counter.
-__device__ __forceinline__ int clone_seed(const EventDev& E, const FindConfigDev& C, int s,
-                                          int layer, int state, int ncand, int cur,
-                                          const SeedRecords& R, HitMatchPair* hm,
-                                          CloneScratch& X, int& upd_out, int lane,
-                                          int* n_records_out = nullptr,
-                                          int* parent_out = nullptr) {
+// Shared-memory scratch of a seed's clone step: the records present (or,
+// then, the best of them in order).
+constexpr int kCloneList = 32;
+struct CloneScratch {
+  int key[kCloneList];  // score_key
+  int id[kCloneList];   // record index, bit 8: a stop (-2), bit 9: a hit
+};
+__device__ __forceinline__ int clone_id(int idx, int hit) {
+  return idx | (hit == -2 ? 256 : 0) | (hit >= 0 ? 512 : 0);
+}
+
+// First half of CandCloner::ProcessSeedRange (mkFit/CandCloner.cc:36-189)
+// for the seeds of a warp, 8 lanes per seed (lane c of them works on
+// candidate c, then on new candidate c): the top records by (score desc,
+// record order), merged with the held-back candidates into the list of new
+// candidates, the best short candidate, and the arena space of the step.
+// All lanes of the warp call it; `on` is false for the lanes of a seed that
+// takes no part. The lanes own the seed.
+__device__ __forceinline__ CloneList clone_rank(const EventDev& E, const FindConfigDev& C, bool on,
+                                                int s, int layer, int ncand, int cur,
+                                                const SeedRecords& R, CloneScratch& X, int lane) {
   constexpr unsigned kFull = 0xffffffffu;
   const CandSoA& B = E.cand[cur];
-  const CandSoA& N = E.cand[cur ^ 1];
   const int M = C.max_cands;
-  upd_out = 0;
-  const int hot0 = E.hot_size[s];
-  // The best short candidate's flag and score, loaded with the seed's
-  // other data rather than one after the other where they are used.
-  const int bs_valid = E.bshort_valid[s];
-  const float bs_score_in = E.bshort.score[s];
+  const int c = lane & 7, g0 = lane & 24, s0 = s * kSlots;
+  const unsigned gmask = 0xffu << g0;
+  const bool is_cand = on && c < ncand;
+  const int hot0 = on ? E.hot_size[s] : 0;
+  const bool bs_valid = on && E.bshort_valid[s];
+  const float bs_in = on ? E.bshort.score[s] : 0.f;
 
-  // Per-candidate values, staged by lane c for candidate c.
-  const int cslot = s * kSlots + (lane < kSlots ? lane : 0);
-  const bool is_cand = lane < ncand;
-  const int c_kind = (is_cand && state == kFinding) ? R.extra_kind(lane) : 0;
-  if (is_cand) {
-    X.cand[8][lane] = __float_as_int(B.score[cslot]);
-    X.cand[9][lane] = __float_as_int(B.par[3 * B.cap + cslot]);
-    X.cand[10][lane] = c_kind;
-    X.cand[0][lane] = B.chg[cslot];
-    X.cand[1][lane] = __float_as_int(B.chi2[cslot]);
-    X.cand[2][lane] = B.last[cslot];
-    X.cand[3][lane] = B.nfound[cslot];
-    X.cand[4][lane] = B.nmiss[cslot];
-    X.cand[5][lane] = B.nover[cslot];
-    X.cand[6][lane] = B.ninside[cslot];
-    X.cand[7][lane] = B.ntail[cslot];
-  }
-
-  constexpr int kPer = (kRecPerSeed + 31) / 32;  // present records per lane, at most
-  // Records present: the mask bits of candidates [0, ncand) (lane c holds
-  // candidate c's mask). In record order they get compacted indices
-  // p = 0 .. n_valid - 1; cincl is the inclusive count up to candidate c.
-  const uint32_t cm = is_cand ? R.mask(lane) : 0u;
-  const int ccount = __popc(cm);
-  int cincl = ccount;
+  // Records present in record order: candidate c's start at place `at`.
+  const uint32_t cm = is_cand ? R.mask(c) : 0u;
+  const int kind = is_cand ? R.extra_kind(c) : 0;
+  int at = __popc(cm);
 #pragma unroll
   for (int off = 1; off < kSlots; off <<= 1) {
-    const int v = __shfl_up_sync(kFull, cincl, off);
-    if (lane >= off) cincl += v;
+    const int v = __shfl_up_sync(kFull, at, off, kSlots);
+    if (c >= off) at += v;
   }
-  const int n_valid = __shfl_sync(kFull, cincl, kSlots - 1);
-  if (n_records_out) *n_records_out = n_valid;
-  // Record index of present record p < n_valid (warp-collective).
-  auto locate = [&](int p) {
-    int c = 0;
-#pragma unroll
-    for (int j = 0; j < kSlots - 1; ++j) c += p >= __shfl_sync(kFull, cincl, j) ? 1 : 0;
-    const uint32_t m = __shfl_sync(kFull, cm, c);
-    const int first = __shfl_sync(kFull, cincl - ccount, c);
-    return c * kRecPerCand + (int)(__fns(m, 0, p - first + 1) & 31u);
-  };
-  const bool mine = lane < n_valid;
-  const int my_idx = locate(lane);
-  Record my_r{0, 0, 0.f, 0.f};
-  if (mine) my_r = R.rec(my_idx);
-
-  // Overlap candidates per parent (consulted at CandCloner.cc:120-124),
-  // filled in hit order as MkFinder does (:1212-1216): lane c considers
-  // candidate c's hit records under the overlap chi2 cut.
-  if (lane < kSlots) {
-    HitMatchPair p;
-    p.reset();
-    uint32_t m = cm & ((1u << kMaxXHits) - 1u);
-    while (m) {
-      const int h = __ffs(m) - 1;
+  const int n_valid = __shfl_sync(kFull, at, kSlots - 1, kSlots);
+  at -= __popc(cm);
+  const unsigned em0 = (__ballot_sync(kFull, kind != 0) >> g0) & 0xffu;
+  const bool listed = n_valid <= kCloneList;
+  if (listed) {
+    // The first two records' loads go out together (a candidate seldom has
+    // more than a hit or two and the hole).
+    uint32_t m = cm;
+    const int h0 = m ? __ffs(m) - 1 : 0;
+    m &= m - 1;
+    const int h1 = m ? __ffs(m) - 1 : 0;
+    Record r0{0, 0, 0.f, 0.f}, r1{0, 0, 0.f, 0.f};
+    if (cm) r0 = R.rec(c * kRecPerCand + h0);
+    if (m) r1 = R.rec(c * kRecPerCand + h1);
+    if (cm) {
+      X.key[at] = score_key(r0.score);
+      X.id[at] = clone_id(c * kRecPerCand + h0, r0.hit);
+    }
+    if (m) {
+      X.key[at + 1] = score_key(r1.score);
+      X.id[at + 1] = clone_id(c * kRecPerCand + h1, r1.hit);
       m &= m - 1;
-      const Record q = R.rec(lane * kRecPerCand + h);
-      if (q.chi2 < C.chi2_cut_overlap) p.consider(q.hit, q.module, q.chi2);
     }
-    hm[lane] = p;
+    for (int p = at + 2; m; m &= m - 1, ++p) {
+      const int idx = c * kRecPerCand + __ffs(m) - 1;
+      const Record r = R.rec(idx);
+      X.key[p] = score_key(r.score);
+      X.id[p] = clone_id(idx, r.hit);
+    }
   }
-
-  // Extras (held-back candidates) in candidate order (MkBuilder.cc:1600-1626).
-  const unsigned extra_mask = __ballot_sync(kFull, c_kind != 0);
-  const int n_extras = __popc(extra_mask);
   __syncwarp();
-
-  if (n_valid == 0) {
-    // hitsForSeed empty (CandCloner.cc:163-172): the extras survive.
-    if (state != kFinding) return -1;
-
-    // Lane i: the i-th extra.
-    int c = 0;
-    if (lane < n_extras) {
-      unsigned mm = extra_mask;
-      for (int k = 0; k < lane; ++k) mm &= mm - 1;
-      c = __ffs(mm) - 1;
-    }
-    copy_par_err(B, N, s, n_extras, c, lane);
-    if (lane < n_extras) {
-      if (parent_out) parent_out[lane] = c;
-      const int src = s * kSlots + c, dst = s * kSlots + lane;
-      // Loads first (see copy_slot).
-      const int chg = B.chg[src], nfound = B.nfound[src], nover = B.nover[src];
-      const int ninside = B.ninside[src], ntail = B.ntail[src], nmiss = B.nmiss[src];
-      const float chi2 = B.chi2[src], score = B.score[src];
-      const bool stop = R.extra_kind(c) == 2;
-      const int last = stop ? R.extra_last(c) : B.last[src];
-      N.chg[dst] = chg;
-      N.chi2[dst] = chi2;
-      N.score[dst] = score;
-      N.nfound[dst] = nfound;
-      N.nover[dst] = nover;
-      N.ninside[dst] = ninside;
-      N.ntail[dst] = ntail;
-      N.last[dst] = last;
-      N.nmiss[dst] = nmiss + (stop ? 1 : 0);
-      R.set_upd(lane, 0);
-    }
-    return n_extras;
-  }
 
   // Top-num_hits records in (score desc, record index asc) order: the
   // reference's std::sort by score; on exact score ties this order is the
-  // stable one. Lane i receives the i-th record and its fields.
+  // stable one. Record p goes to the place given by the count of those
+  // before it.
   const int num_hits = min(n_valid, M);
-  const bool has_rec = lane < num_hits;
-  int my_rec = 0, r_hit = 0, r_module = 0;
-  float r_score = 0.f, r_chi2 = 0.f;
-  if (n_valid <= 32) {
-    // Lane p holds present record p: rank each against all others, place
-    // the first num_hits by rank.
-    const int key = mine ? score_key(my_r.score) : INT_MIN;
-    int rank = 0;
-    for (int j = 0; j < n_valid; ++j) {
-      const int kj = __shfl_sync(kFull, key, j);
-      rank += (kj > key) || (kj == key && j < lane);
-    }
-    if (mine && rank < num_hits) {
-      X.rec[rank] = my_idx;
-      X.hit[rank] = my_r.hit;
-      X.score[rank] = my_r.score;
-      X.chi2[rank] = my_r.chi2;
-      X.module[rank] = my_r.module;
-    }
-    __syncwarp();
-    if (has_rec) {
-      my_rec = X.rec[lane];
-      r_hit = X.hit[lane];
-      r_score = X.score[lane];
-      r_chi2 = X.chi2[lane];
-      r_module = X.module[lane];
-    }
-  } else {
-    // More records than lanes: num_hits rounds of a warp arg-max over the
-    // compacted indices (their order is the record order).
-    int key[kPer];
+  constexpr int kPer = kCloneList / kSlots;
+  int key[kPer], id[kPer], rank[kPer];
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const int p = lane + 32 * k;
-      const int idx = locate(p);
-      key[k] = p < n_valid ? score_key(R.rec(idx).score) : INT_MIN;
+  for (int k = 0; k < kPer; ++k) {
+    const int p = c + kSlots * k;
+    rank[k] = kCloneList;
+    if (listed && kSlots * k < n_valid) {
+      const bool in = p < n_valid;
+      key[k] = in ? X.key[p] : kNoKey;
+      id[k] = in ? X.id[p] : 0;
+      int r = 0;
+      for (int j = 0; j < n_valid; ++j) {
+        const int kj = X.key[j];
+        r += (kj > key[k]) || (kj == key[k] && j < p);
+      }
+      if (in) rank[k] = r;
     }
-    bool left[kPer];
+  }
+  __syncwarp();
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) left[k] = lane + 32 * k < n_valid;
-    int my_p = 0;
+  for (int k = 0; k < kPer; ++k)
+    if (rank[k] < num_hits) {
+      X.key[rank[k]] = key[k];
+      X.id[rank[k]] = id[k];
+    }
+  if (!listed) {
+    // More records than places: num_hits rounds, each the best of what is
+    // left (lane c looks through candidate c's records).
+    uint32_t left = cm;
     for (int i = 0; i < num_hits; ++i) {
-      int best = INT_MIN, bidx = INT_MAX;
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        const int p = lane + 32 * k;
-        if (left[k] && (key[k] > best || (key[k] == best && p < bidx))) {
-          best = key[k];
-          bidx = p;
+      int bk = kNoKey, bi = INT_MAX, bv = 0;
+      for (uint32_t m = left; m; m &= m - 1) {
+        const int idx = c * kRecPerCand + __ffs(m) - 1;
+        const Record r = R.rec(idx);
+        if (score_key(r.score) > bk) {
+          bk = score_key(r.score);
+          bi = idx;
+          bv = clone_id(idx, r.hit);
         }
       }
+      int wk = bk, wi = bi;
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const int ob = __shfl_xor_sync(kFull, best, off);
-        const int oi = __shfl_xor_sync(kFull, bidx, off);
-        if (ob > best || (ob == best && oi < bidx)) {
-          best = ob;
-          bidx = oi;
+      for (int off = kSlots / 2; off > 0; off >>= 1) {
+        const int ok = __shfl_xor_sync(gmask, wk, off, kSlots);
+        const int oi = __shfl_xor_sync(gmask, wi, off, kSlots);
+        if (ok > wk || (ok == wk && oi < wi)) {
+          wk = ok;
+          wi = oi;
         }
       }
-      if (lane == i) my_p = bidx;
-#pragma unroll
-      for (int k = 0; k < kPer; ++k)
-        if (lane + 32 * k == bidx) left[k] = false;
-    }
-    my_rec = locate(my_p);
-    if (has_rec) {
-      const Record q = R.rec(my_rec);
-      r_hit = q.hit;
-      r_score = q.score;
-      r_chi2 = q.chi2;
-      r_module = q.module;
+      if (bi == wi) {
+        X.key[i] = bk;
+        X.id[i] = bv;
+        left &= ~(1u << (bi - c * kRecPerCand));
+      }
     }
   }
+  __syncwarp();
 
-  // Build the new candidate list (logic of ProcessSeedRange); lane i keeps
-  // new candidate i.
-  NewCand nc{0, 0, 0.f, -1, 0.f, 0};
-  int n_pushed = 0;
-  float bs_score = bs_valid ? bs_score_in : -1e16f;  // getScoreWorstPossible
+  // The new candidate list. The best short candidate's score decides
+  // whether a stop (-2) record replaces it.
+  CloneList out{0, n_valid, 0, 0, 0, -1, 0, false};
   int bs_from = -1;
-  if (extra_mask == 0) {
-    // No extras: the new candidates are the records in order, less the
-    // stop (-2) records, of which the first (best) may replace the best
-    // short candidate. All lanes at once.
-    const bool is_stop = has_rec && r_hit == -2;
-    const unsigned stop_mask = __ballot_sync(kFull, is_stop);
-    const unsigned push_mask = __ballot_sync(kFull, has_rec && !is_stop);
-    n_pushed = __popc(push_mask);
-    if (stop_mask) {
-      const int f = __ffs(stop_mask) - 1;
-      const float sc = __shfl_sync(kFull, r_score, f);
-      const int rec = __shfl_sync(kFull, my_rec, f);
-      if (sc > bs_score) {
-        bs_score = sc;
-        bs_from = rec;
+  float bs_score = bs_valid ? bs_in : -1e16f;  // getScoreWorstPossible
+  const bool has = c < num_hits;
+  const int my_id = has ? X.id[c] : 0;
+  const unsigned stop_m = (__ballot_sync(kFull, has && (my_id & 256)) >> g0) & 0xffu;
+  const unsigned push_m = (__ballot_sync(kFull, has && !(my_id & 256)) >> g0) & 0xffu;
+  if (n_valid == 0) {
+    // hitsForSeed empty (CandCloner.cc:163-172): the extras survive.
+    out.n = __popc(em0);
+    out.parent = c < out.n ? (int)__fns(em0, 0, c + 1) : 0;
+  } else if (em0 == 0) {
+    // No extras: the records in order, less the stops, of which the first
+    // (best) may replace the best short candidate. All lanes at once.
+    out.n = __popc(push_m);
+    if (stop_m) {
+      const int f = __ffs(stop_m) - 1;
+      if (key_score(X.key[f]) > bs_score) bs_from = X.id[f] & 255;
+    }
+    out.rec = X.id[c < out.n ? (stop_m ? (int)__fns(push_m, 0, c + 1) : c) : 0];
+    out.parent = (out.rec & 255) / kRecPerCand;
+  } else {
+    // Extras and records in turn, the same in every lane of the seed.
+    const float my_score = is_cand ? B.score[s0 + c] : 0.f;
+    unsigned em = em0;
+    auto push = [&](int rec, int parent) {
+      if (c == out.n) {
+        out.rec = rec;
+        out.parent = parent;
       }
-    }
-    const int src = stop_mask ? (int)__fns(push_mask, 0, lane + 1) & 31 : lane;
-    const int idx = __shfl_sync(kFull, my_rec, src);
-    const int hit = __shfl_sync(kFull, r_hit, src);
-    const float score = __shfl_sync(kFull, r_score, src);
-    const float chi2hit = __shfl_sync(kFull, r_chi2, src);
-    const int module = __shfl_sync(kFull, r_module, src);
-    const int parent = idx / kRecPerCand;
-    if (lane < n_pushed) {
-      const float ppt = fabsf(1.f / __int_as_float(X.cand[9][parent]));
-      int ov = -1;
-      if (ppt > C.pt_cut_overlap && hit >= 0) ov = hm[parent].find(hit, module);
-      nc = NewCand{parent, hit, chi2hit, ov, score, 0};
-    }
-  }
-  auto push = [&](const NewCand& v) {
-    if (lane == n_pushed) nc = v;
-    ++n_pushed;
-  };
-  unsigned em = extra_mask;  // extras not yet taken, in candidate order
-  // With extras: sequentially, identically in every lane from the
-  // broadcast values.
-  for (int ih = 0; ih < (extra_mask ? num_hits : 0); ++ih) {
-    const int idx = __shfl_sync(kFull, my_rec, ih);
-    const int hit = __shfl_sync(kFull, r_hit, ih);
-    const float score = __shfl_sync(kFull, r_score, ih);
-    const float chi2hit = __shfl_sync(kFull, r_chi2, ih);
-    const int module = __shfl_sync(kFull, r_module, ih);
-    const int parent = idx / kRecPerCand;
-    if (hit == -2) {
-      if (score > bs_score) {
-        bs_score = score;
-        bs_from = idx;
+      ++out.n;
+    };
+    for (int ih = 0; ih < num_hits; ++ih) {
+      const int rid = X.id[ih];
+      const float score = key_score(X.key[ih]);
+      if (rid & 256) {
+        if (score > bs_score) {
+          bs_score = score;
+          bs_from = rid & 255;
+        }
+        continue;
       }
-      continue;
+      while (em && out.n < M) {
+        const int e = __ffs(em) - 1;
+        if (!(__shfl_sync(gmask, my_score, e, kSlots) > score)) break;
+        push(-1, e);
+        em &= em - 1;
+      }
+      if (out.n >= M) break;
+      push(rid, (rid & 255) / kRecPerCand);
     }
-    while (em && n_pushed < M) {
-      const int c = __ffs(em) - 1;
-      if (!(__int_as_float(X.cand[8][c]) > score)) break;
-      push(NewCand{c, 0, 0.f, -1, 0.f, X.cand[10][c]});
-      em &= em - 1;
-    }
-    if (n_pushed >= M) break;
-    int ov = -1;
-    const float ppt = fabsf(1.f / __int_as_float(X.cand[9][parent]));
-    if (ppt > C.pt_cut_overlap && hit >= 0) ov = hm[parent].find(hit, module);
-    push(NewCand{parent, hit, chi2hit, ov, score, 0});
+    for (; em && out.n < M; em &= em - 1) push(-1, __ffs(em) - 1);
   }
-  while (em && n_pushed < M) {
-    const int c = __ffs(em) - 1;
-    push(NewCand{c, 0, 0.f, -1, 0.f, X.cand[10][c]});
-    em &= em - 1;
-  }
+  // Lane i < n: candidate i's record (held-back copies have none).
+  const bool mine = c < out.n;
+  const bool from_rec = mine && n_valid > 0 && out.rec >= 0;
+  const bool hit = from_rec && (out.rec & 512);
+  out.rec = from_rec ? out.rec & 255 : 0;
+  out.kind = __shfl_sync(kFull, kind, out.parent, kSlots);
+  if (from_rec || !mine) out.kind = 0;
 
-  // The parents' parameters and covariances are loaded now, so the loads
-  // overlap the node and best-short bookkeeping (stored at the end).
-  float pe[7];
-  load_par_err(B, s, n_pushed, nc.parent, lane, pe);
+  // The overlap hit (CandCloner.cc:120-124): the parent's hit records under
+  // the overlap chi2 cut, considered in hit order as MkFinder does
+  // (:1212-1216). A record's own hit never pairs with itself, so a parent
+  // without another one needs no look.
+  const uint32_t pm = __shfl_sync(kFull, cm, out.parent, kSlots) & ((1u << kMaxXHits) - 1u);
+  if (hit) {
+    const int h = out.rec - out.parent * kRecPerCand;
+    if ((pm & ~(1u << h)) && fabsf(1.f / B.par[3 * B.cap + s0 + out.parent]) > C.pt_cut_overlap) {
+      HitMatchPair p;
+      p.reset();
+      int module = 0;
+      for (uint32_t m = pm; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const Record q = R.rec(out.parent * kRecPerCand + k);
+        if (k == h) module = q.module;
+        if (q.chi2 < C.chi2_cut_overlap) p.consider(k, q.module, q.chi2);
+      }
+      const int f = p.find(h, module);
+      if (f >= 0) out.ov = out.parent * kRecPerCand + (f ? p.hit[1] : p.hit[0]);
+    }
+  }
+  out.upd = hit;
+
   // Arena nodes of this step, one allocation for the seed: the best short
   // candidate's hole node first, then one or two nodes per new candidate
-  // with a hit, in candidate order.
-  const bool own = lane < n_pushed && !nc.is_extra;
-  const int n_nodes = own ? 1 + (nc.ov >= 0) : 0;
-  int node_off = n_nodes;
+  // with a record, in candidate order.
+  const int own = from_rec ? 1 + (out.ov >= 0) : 0;
+  int nodes = own;
 #pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int v = __shfl_up_sync(kFull, node_off, off);
-    if (lane >= off) node_off += v;
+  for (int off = 1; off < kSlots; off <<= 1) {
+    const int v = __shfl_up_sync(kFull, nodes, off, kSlots);
+    if (c >= off) nodes += v;
   }
-  const int nodes_total = __shfl_sync(kFull, node_off, 31) + (bs_from >= 0);
-  node_off -= n_nodes;
-  if (lane == 0 && nodes_total) E.hot_size[s] = hot0 + nodes_total;
-  const int node_base = hot0 + (bs_from >= 0);
+  const int total = __shfl_sync(kFull, nodes, kSlots - 1, kSlots) + (bs_from >= 0);
+  if (on && c == 0 && total) E.hot_size[s] = hot0 + total;
+  out.node = hot0 + (bs_from >= 0) + nodes - own;
 
-  // Best short candidate (a -2 record scoring above the current best).
+  // Best short candidate (a -2 record scoring above the current best): the
+  // parent with the stop as its last node; its state by all 8 lanes. Loads
+  // first (see copy_slot).
   if (bs_from >= 0) {
-    const int parent = bs_from / kRecPerCand;
-    const int src = s * kSlots + parent;
-    if (lane < 27) {
-      if (lane < 6) E.bshort.par[lane * E.bshort.cap + s] = B.par[lane * B.cap + src];
-      else E.bshort.err[(lane - 6) * E.bshort.cap + s] = B.err[(lane - 6) * B.cap + src];
+    const int src = s0 + bs_from / kRecPerCand;
+    float v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int e = c + kSlots * k;
+      if (e < 27) v[k] = (e < 6 ? B.par + e * B.cap : B.err + (e - 6) * B.cap)[src];
     }
-    if (lane == 0) {
+    if (c == 0) {
       int nfound = B.nfound[src], nmiss = B.nmiss[src], nin = B.ninside[src], ntl = B.ntail[src];
       float chi2 = B.chi2[src];
       const int chg = B.chg[src], nover = B.nover[src], last = B.last[src];
+      const float score = R.rec(bs_from).score;
       add_hit_counts(-2, 0.f, nfound, nmiss, nin, ntl, chi2);
-      E.bshort.last[s] = arena_put(E, s, node_base - 1, -2, layer, 0.f, last);
+      E.bshort.last[s] = arena_put(E, s, hot0, -2, layer, 0.f, last);
       E.bshort.chg[s] = chg;
       E.bshort.chi2[s] = chi2;
-      E.bshort.score[s] = bs_score;
+      E.bshort.score[s] = score;
       E.bshort.nfound[s] = nfound;
       E.bshort.nmiss[s] = nmiss;
       E.bshort.nover[s] = nover;
@@ -972,53 +854,70 @@ __device__ __forceinline__ int clone_seed(const EventDev& E, const FindConfigDev
       E.bshort.ntail[s] = ntl;
       E.bshort_valid[s] = 1;
     }
-  }
-
-  // Materialize the new candidates into the other buffer: parameters and
-  // covariance by all lanes, counters and hit-on-track nodes of new
-  // candidate i by lane i.
-  store_par_err(N, s, n_pushed, lane, pe);
-  if (lane < n_pushed) {
-    if (parent_out) parent_out[lane] = nc.parent;
-    const int pc = nc.parent, dst = s * kSlots + lane;
-    int nfound = X.cand[3][pc], nmiss = X.cand[4][pc], nin = X.cand[6][pc], ntl = X.cand[7][pc];
-    int nover = X.cand[5][pc];
-    float chi2 = __int_as_float(X.cand[1][pc]);
-    int last = X.cand[2][pc];
-    float score = __int_as_float(X.cand[8][pc]);
-    int upd = 0;
-    if (nc.is_extra) {
-      if (nc.is_extra == 2) {
-        last = R.extra_last(nc.parent);
-        ++nmiss;
-      }
-    } else {
-      const int pos = node_base + node_off;
-      add_hit_counts(nc.hit, nc.chi2hit, nfound, nmiss, nin, ntl, chi2);
-      last = arena_put(E, s, pos, nc.hit, layer, nc.chi2hit, last);
-      score = nc.score;
-      if (nc.ov >= 0) {
-        const HitMatchPair& p = hm[nc.parent];
-        add_hit_counts(p.hit[nc.ov], p.chi2[nc.ov], nfound, nmiss, nin, ntl, chi2);
-        last = arena_put(E, s, pos + 1, p.hit[nc.ov], layer, p.chi2[nc.ov], last);
-        ++nover;
-      }
-      // UpdateWithLastHit uses the last hit added: the overlap hit if any.
-      if (nc.hit >= 0) upd = 1 + (nc.ov >= 0 ? hm[nc.parent].hit[nc.ov] : nc.hit);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int e = c + kSlots * k;
+      if (e < 27)
+        (e < 6 ? E.bshort.par + e * E.bshort.cap : E.bshort.err + (e - 6) * E.bshort.cap)[s] = v[k];
     }
-    N.chg[dst] = X.cand[0][pc];
-    N.chi2[dst] = chi2;
-    N.score[dst] = score;
-    N.last[dst] = last;
-    N.nfound[dst] = nfound;
-    N.nmiss[dst] = nmiss;
-    N.nover[dst] = nover;
-    N.ninside[dst] = nin;
-    N.ntail[dst] = ntl;
-    R.set_upd(lane, upd);
-    upd_out = upd;
   }
-  return n_pushed;
+  return out;
+}
+
+// Second half, by lane i < l.n of the seed's 8: new candidate i written
+// into the other buffer -- counters and hit-on-track nodes, and the
+// parent's parameters and covariance unless an update follows, which reads
+// them from the parent and writes the updated ones (copy_all: always).
+// Returns its update code: 1 + the index in the layer of the last hit added
+// (the overlap hit if any), 0 for none.
+__device__ __forceinline__ int clone_write(const EventDev& E, int s, int layer, int cur,
+                                           const SeedRecords& R, const CloneList& l, int i,
+                                           bool copy_all) {
+  const CandSoA& B = E.cand[cur];
+  const CandSoA& N = E.cand[cur ^ 1];
+  const int src = s * kSlots + l.parent, dst = s * kSlots + i;
+  Record r{0, 0, 0.f, 0.f}, q{0, 0, 0.f, 0.f};
+  if (!l.kind) r = R.rec(l.rec);
+  if (l.ov >= 0) q = R.rec(l.ov);
+  // Loads first (see copy_slot).
+  const int chg = B.chg[src];
+  int nfound = B.nfound[src], nmiss = B.nmiss[src], nover = B.nover[src];
+  int nin = B.ninside[src], ntl = B.ntail[src], last = B.last[src];
+  float chi2 = B.chi2[src], score = B.score[src];
+  if (copy_all || !l.upd) {
+    float par[6], err[21];
+    load_state(B, src, par, err);
+    store_state(N, dst, par, err);
+  }
+  int upd = 0;
+  if (l.kind) {
+    if (l.kind == 2) {
+      last = R.extra_last(l.parent);
+      ++nmiss;
+    }
+  } else {
+    add_hit_counts(r.hit, r.chi2, nfound, nmiss, nin, ntl, chi2);
+    last = arena_put(E, s, l.node, r.hit, layer, r.chi2, last);
+    score = r.score;
+    int hit = r.hit;
+    if (l.ov >= 0) {
+      add_hit_counts(q.hit, q.chi2, nfound, nmiss, nin, ntl, chi2);
+      last = arena_put(E, s, l.node + 1, q.hit, layer, q.chi2, last);
+      ++nover;
+      hit = q.hit;
+    }
+    if (l.upd) upd = 1 + hit;
+  }
+  N.chg[dst] = chg;
+  N.chi2[dst] = chi2;
+  N.score[dst] = score;
+  N.last[dst] = last;
+  N.nfound[dst] = nfound;
+  N.nmiss[dst] = nmiss;
+  N.nover[dst] = nover;
+  N.ninside[dst] = nin;
+  N.ntail[dst] = ntl;
+  return upd;
 }
 
 // Candidate score for the final merge: getScoreCand with default arguments

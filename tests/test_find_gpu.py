@@ -925,6 +925,89 @@ def test_clone_worker_matches_reference(gpu_ctx, reflib):
     assert n_ovl > 50 and n_held > 50 and moved.sum() > 50
 
 
+def restate_clone(inp, s, m, cfg):
+    """CandCloner::ProcessSeedRange (mkFit/CandCloner.cc:36-189) for seed s of
+    `inp` in Python: [(parent, hit or NO_HIT, overlap hit or -1, score)] and
+    the best short candidate (score, parent) or None if it stays."""
+    from mkfit_b200.finder import NO_HIT
+    c0, nc = 8 * s, int(inp["n_cands"][s])
+    recs, pairs = [], {}
+    for c in range(nc):
+        k, p = c0 + c, dict(hit=[-1, -1], module=[-1, -1], chi2=[1e9, 1e9])
+        for j in range(inp["n_rec"][k]):
+            h, md = int(inp["rec_hit"][k, j]), int(inp["rec_module"][k, j])
+            x = float(inp["rec_chi2"][k, j])
+            recs.append((float(inp["rec_score"][k, j]), c, h, md))
+            if h < 0 or x >= cfg["chi2_cut_overlap"]:
+                continue
+            if md in p["module"]:
+                t = p["module"].index(md)
+                if x >= p["chi2"][t]:
+                    continue
+            else:
+                t = 0 if p["chi2"][0] > p["chi2"][1] else 1
+                if x >= p["chi2"][t]:
+                    continue
+            p["hit"][t], p["module"][t], p["chi2"][t] = h, md, x
+        pairs[c] = p
+    extras = [c for c in range(nc) if inp["held_back"][c0 + c]]
+    recs.sort(key=lambda r: -r[0])
+    out, short, best = [], None, (float(inp["bshort_score"][s]) if inp["bshort_valid"][s] else -1e16)
+    if not recs:
+        return [(c, NO_HIT, -1, float(inp["score"][c0 + c])) for c in extras], None
+    for score, c, h, md in recs[:m]:
+        if h == -2:
+            if score > best:
+                best, short = score, (score, c)
+            continue
+        while extras and len(out) < m and float(inp["score"][c0 + extras[0]]) > score:
+            e = extras.pop(0)
+            out.append((e, NO_HIT, -1, float(inp["score"][c0 + e])))
+        if len(out) >= m:
+            break
+        ov, p = -1, pairs[c]
+        if h >= 0 and abs(np.float32(1) / inp["par"][3][c0 + c]) > cfg["pt_cut_overlap"]:
+            if md in p["module"]:
+                ov = p["hit"][1 - p["module"].index(md)]
+            else:
+                ov = p["hit"][0 if p["chi2"][0] <= p["chi2"][1] else 1]
+        out.append((c, h, ov, score))
+    while extras and len(out) < m:
+        e = extras.pop(0)
+        out.append((e, NO_HIT, -1, float(inp["score"][c0 + e])))
+    return out, short
+
+
+@pytest.mark.parametrize("m,n_seeds", [(1, 1), (2, 31), (3, 33), (6, 700), (8, 257)])
+def test_clone_worker_matches_restatement(gpu_ctx, m, n_seeds):
+    """The clone step (ranking and writing) against its restatement: the new
+    candidates in order, their parents' states bit for bit, and the best
+    short candidate, for every list length."""
+    from mkfit_b200.finder import NO_HIT
+    inp = clone_inputs(n_seeds, np.random.default_rng(100 + m), m)
+    cfg = FindConfig(max_cands=m, chi2_cut=30.0, zero_c2=True)
+    cuts = dict(chi2_cut_overlap=cfg.c.chi2_cut_overlap, pt_cut_overlap=cfg.c.pt_cut_overlap)
+    got = Finder(gpu_ctx, cfg).clone_seeds(4, inp)
+    for s in range(n_seeds):
+        exp, short = restate_clone(inp, s, m, cuts)
+        assert got["n_cands"][s] == len(exp), s
+        for i, (c, h, ov, score) in enumerate(exp):
+            k, src = 8 * s + i, 8 * s + c
+            assert (got["parent"][k], got["hit"][k], got["overlap_hit"][k]) == (c, h, ov), (s, i)
+            assert got["score"][k] == np.float32(score)
+            assert got["update_hit"][k] == (-1 if h < 0 else ov if ov >= 0 else h)
+            np.testing.assert_array_equal(got["par"][:, k], inp["par"][:, src])
+            np.testing.assert_array_equal(got["err"][:, k], inp["err"][:, src])
+            stop = h == NO_HIT and inp["held_back"][src] == 2
+            assert got["nfound"][k] == inp["nfound"][src] + (h >= 0) + (ov >= 0)
+            assert got["nmiss"][k] == inp["nmiss"][src] + (h < 0 and (h != NO_HIT or stop))
+        if short is None:
+            assert got["bshort_valid"][s] == (inp["bshort_valid"][s] != 0)
+        else:
+            assert got["bshort_valid"][s] and got["bshort_score"][s] == np.float32(short[0])
+            assert got["bshort_nfound"][s] == inp["nfound"][8 * s + short[1]]
+
+
 def test_device_seed_import_equals_host(gpu_ctx):
     """The device seed import (region, eta order and initial candidates made
     on the device) and the host one (the upload's worker threads) give the
