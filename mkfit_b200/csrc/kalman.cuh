@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include "flat_math.cuh"
 #include "generated_ops.cuh"
 
 namespace mkfg {
@@ -108,6 +109,22 @@ __device__ __forceinline__ float hypot_f(float x, float y) {
   return (float)sqrt(dx * dx + dy * dy);
 }
 
+// The plain form of the step's arithmetic (flat_math.cuh).
+struct ExactMath {
+  static constexpr bool kPlain = true;
+  __device__ __forceinline__ void see(float) {}
+  __device__ __forceinline__ void see_wide(float) {}
+  __device__ __forceinline__ bool ok() const { return true; }
+  __device__ __forceinline__ static float rcp(float b) { return 1.f / b; }
+  __device__ __forceinline__ static float div(float a, float b) { return a / b; }
+  __device__ __forceinline__ static float div_const(float a, float b, float) { return a / b; }
+  __device__ __forceinline__ static float sqrt(float x) { return sqrtf(x); }
+  __device__ __forceinline__ static void sincos(float x, float* s, float* c) { f_sincos(x, s, c); }
+  __device__ __forceinline__ static float log(float x) { return f_log(x); }
+  __device__ __forceinline__ static float hypot(float x, float y) { return hypot_f(x, y); }
+  __device__ __forceinline__ static float inv_det(double det) { return (float)(1.0 / det); }
+};
+
 // Magnetic field model (Config.h:434-437).
 __device__ __forceinline__ float bfield_zr(float z, float r) {
   return (kMagB0 * z * z + kMagB1 * z + kMagC1) * (kMagA * r * r + 1.f);
@@ -130,38 +147,69 @@ __device__ __forceinline__ float squash_phi(float phi) {
 //------------------------------------------------------------------------------
 // Helix to radius r: 5 fixed iterations with arc-length derivative tracking.
 // Restates helixAtRFromIterativeCCS_impl (mkFit/PropagationMPlex.icc:5-246).
-// Returns the fail flag (1 when the step would approach the apex).
+// Returns the fail flag (1 when the step would approach the apex), and the
+// sine of theta for the material effects.
 //------------------------------------------------------------------------------
-__device__ __forceinline__ int helix_to_r(const float (&in)[6], int chg, float r, bool param_b,
-                                          float (&out)[6], float (&J)[36]) {
+// k = charge * 100 / (-sol * B) of a unit charge in the constant field.
+constexpr float kCurv1 = 100.f / (-kSol * kBfield);
+constexpr float kCurvInv1 = 1.f / kCurv1;
+
+// The curvature constant k and its inverse.
+template <class F>
+__device__ __forceinline__ void curvature(F& m, int chg, bool param_b, float z, float r, float& k,
+                                          float& kinv) {
+  if (!param_b && (chg == 1 || chg == -1)) {
+    k = chg > 0 ? kCurv1 : -kCurv1;
+    kinv = chg > 0 ? kCurvInv1 : -kCurvInv1;
+    return;
+  }
+  const float bf = param_b ? bfield_zr(z, r) : kBfield;
+  const float d = -kSol * bf;
+  m.see(d);
+  k = F::div(float(chg) * 100.f, d);
+  m.see(k);
+  kinv = F::rcp(k);
+}
+
+template <class F>
+__device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, float r, bool param_b,
+                                          float (&out)[6], float (&J)[36], float& sinT) {
 #pragma unroll
   for (int i = 0; i < 36; ++i) J[i] = 0.f;
   int fail = 0;
 
-  float r0 = hipo(in[0], in[1]);
-  const float bf = param_b ? bfield_zr(in[2], r0) : kBfield;
-  const float k = float(chg) * 100.f / (-kSol * bf);
+  float r02 = in[0] * in[0] + in[1] * in[1];
+  m.see(r02);
+  float r0 = F::sqrt(r02);
+  float k, kinv;
+  curvature(m, chg, param_b, in[2], r0, k, kinv);
 
   const float xin = in[0], yin = in[1], ipt = in[3], phiin = in[4], theta = in[5];
-  const float kinv = 1.f / k;
-  const float pt = 1.f / ipt;
+  m.see(ipt);
+  const float pt = F::rcp(ipt);
 
   float D = 0.f, cosa = 0.f, sina = 0.f, cosah = 0.f, sinah = 0.f, id = 0.f;
   float cosPorT, sinPorT;
-  f_sincos(phiin, &sinPorT, &cosPorT);
+  m.sincos(phiin, &sinPorT, &cosPorT);
   float pxin = cosPorT * pt;
   float pyin = sinPorT * pt;
 
-  float dDdx = r0 > 0.f ? -xin / r0 : 0.f;
-  float dDdy = r0 > 0.f ? -yin / r0 : 0.f;
+  float dDdx = r0 > 0.f ? F::div(-xin, r0) : 0.f;
+  float dDdy = r0 > 0.f ? F::div(-yin, r0) : 0.f;
   float dDdipt = 0.f;
   float dDdphi = 0.f;
 
   float ox = in[0], oy = in[1];
 #pragma unroll
   for (int it = 0; it < kNiter; ++it) {
-    r0 = hipo(ox, oy);
-    const float oodotp = r0 * pt / (pxin * ox + pyin * oy);
+    if (it > 0) {
+      r02 = ox * ox + oy * oy;
+      m.see(r02);
+      r0 = F::sqrt(r02);
+    }
+    const float dot = pxin * ox + pyin * oy;
+    m.see(dot);
+    const float oodotp = F::div(r0 * pt, dot);
     if (oodotp > 5.0f || oodotp < 0) {
       id = 0.0f;
       fail = 1;
@@ -174,9 +222,13 @@ __device__ __forceinline__ int helix_to_r(const float (&in)[6], int chg, float r
     cosa = 1.f - 2.f * sinah * sinah;
     sina = 2.f * sinah * cosah;
 
-    if (it + 1 != kNiter) {
+    // Far from the target radius (the first steps) the factor 1 / r0 of
+    // every derivative term is 0: FlatMath, whose numbers are finite, skips
+    // them there.
+    const bool near_r = r0 > 0.f && fabsf(r - r0) < 0.0001f;
+    if (it + 1 != kNiter && (F::kPlain || near_r)) {
       const float x = ox, y = oy;
-      const float oor0 = (r0 > 0.f && fabsf(r - r0) < 0.0001f) ? 1.f / r0 : 0.f;
+      const float oor0 = near_r ? F::rcp(r0) : 0.f;
       const float dadipt = id * kinv;
       const float dadx = -x * ipt * kinv * oor0;
       const float dady = -y * ipt * kinv * oor0;
@@ -219,9 +271,10 @@ __device__ __forceinline__ int helix_to_r(const float (&in)[6], int chg, float r
   J[1 * 6 + 3] = k * (sinPorT * (ipt * dadipt * cosa - sina) + cosPorT * (ipt * dadipt * sina - (1.f - cosa))) * pt * pt;
   J[1 * 6 + 4] = k * (sinPorT * dadphi * cosa + cosPorT * dadphi * sina + sinPorT * cosa + cosPorT * sina - sinPorT) * pt;
 
-  float cosT, sinT;
-  f_sincos(theta, &sinT, &cosT);
-  const float isinT = 1.f / sinT;
+  float cosT;
+  m.sincos(theta, &sinT, &cosT);
+  m.see(sinT);
+  const float isinT = F::rcp(sinT);
 
   out[0] = ox;
   out[1] = oy;
@@ -251,8 +304,10 @@ __device__ __forceinline__ int helix_to_r(const float (&in)[6], int chg, float r
 //------------------------------------------------------------------------------
 // Helix to plane z (endcap). Restates helixAtZ (mkFit/PropagationMPlex.cc:604-712).
 //------------------------------------------------------------------------------
-__device__ __forceinline__ void helix_to_z(const float (&in)[6], int chg, float zout, bool param_b,
-                                           float (&out)[6], float (&J)[36]) {
+template <class F>
+__device__ __forceinline__ void helix_to_z(F& m, const float (&in)[6], int chg, float zout,
+                                           bool param_b, float (&out)[6], float (&J)[36],
+                                           float& sinT, float& cosT) {
 #pragma unroll
   for (int i = 0; i < 36; ++i) J[i] = 0.f;
   J[0 * 6 + 0] = 1.f;
@@ -262,16 +317,17 @@ __device__ __forceinline__ void helix_to_z(const float (&in)[6], int chg, float 
   J[5 * 6 + 5] = 1.f;
 
   const float zin = in[2], ipt = in[3], phiin = in[4], theta = in[5];
-  const float bf = param_b ? bfield_zr(zin, hipo(in[0], in[1])) : kBfield;
-  const float k = float(chg) * 100.f / (-kSol * bf);
-  const float kinv = 1.f / k;
-  const float pt = 1.f / ipt;
+  float k, kinv;
+  curvature(m, chg, param_b, zin, param_b ? hipo(in[0], in[1]) : 0.f, k, kinv);
+  m.see(ipt);
+  const float pt = F::rcp(ipt);
 
-  float cosP, sinP, cosT, sinT;
-  f_sincos(phiin, &sinP, &cosP);
-  f_sincos(theta, &sinT, &cosT);
-  const float tanT = sinT / cosT;
-  const float icos2T = 1.f / (cosT * cosT);
+  float cosP, sinP;
+  m.sincos(phiin, &sinP, &cosP);
+  m.sincos(theta, &sinT, &cosT);
+  m.see(cosT);
+  const float tanT = F::div(sinT, cosT);
+  const float icos2T = F::rcp(cosT * cosT);
   const float pxin = cosP * pt;
   const float pyin = sinP * pt;
 
@@ -312,36 +368,47 @@ __device__ __forceinline__ void helix_to_z(const float (&in)[6], int chg, float 
 // (mkFit/PropagationMPlex.cc:716-767): updates C[3][3], C[4][4], C[5][5] of
 // the (pre-similarity) covariance and 1/pT of the propagated parameters.
 //------------------------------------------------------------------------------
-__device__ __forceinline__ void material_effects(float radL, float xi, float prop_sign, bool is_barrel,
+// sinT, cosT: of par[5] (cosT read in the endcaps only). The operands of the
+// divisions and roots are bounded by 1/pT and sinT (cosT), which are seen
+// here again.
+template <class F>
+__device__ __forceinline__ void material_effects(F& m, float radL, float xi, float prop_sign,
+                                                 bool is_barrel, float sinT, float cosT,
                                                  float (&C)[21], float (&par)[6]) {
   if (radL < 1e-13f) return;
-  const float theta = par[5];
-  const float pt = 1.f / par[3];
-  const float p = pt / f_sin(theta);
+  m.see(par[3]);
+  m.see(sinT);
+  const float pt = F::rcp(par[3]);
+  const float p = F::div(pt, sinT);
   const float p2 = p * p;
   constexpr float mpi = 0.140f;
   constexpr float mpi2 = mpi * mpi;
-  const float beta2 = p2 / (p2 + mpi2);
-  const float beta = sqrtf(beta2);
-  const float invCos = is_barrel ? p / pt : 1.f / fabsf(f_cos(theta));
+  const float beta2 = F::div(p2, p2 + mpi2);
+  const float beta = F::sqrt(beta2);
+  const float invCos = is_barrel ? F::div(p, pt) : F::rcp(fabsf(cosT));
   radL = radL * invCos;
   if (radL < 1e-13f) return;
-  const float thetaMSC = 0.0136f * (1.f + 0.038f * f_log(radL)) / (beta * p);
+  const float thetaMSC = F::div(0.0136f * (1.f + 0.038f * m.log(radL)), beta * p);
   const float thetaMSC2 = thetaMSC * thetaMSC * radL;
   C[14] += thetaMSC2;  // (4,4)
   C[20] += thetaMSC2;  // (5,5)
-  const float gamma2 = (p2 + mpi2) / mpi2;
-  const float gamma = sqrtf(gamma2);
+  constexpr float impi2 = 1.f / mpi2, impi = 1.f / mpi;
+  const float gamma2 = F::div_const(p2 + mpi2, mpi2, impi2);
+  const float gamma = F::sqrt(gamma2);
   constexpr float me = 0.0005f;
-  const float wmax = 2.f * me * beta2 * gamma2 / (1.f + 2.f * gamma * me / mpi + me * me / (mpi * mpi));
+  const float wmax = F::div(2.f * me * beta2 * gamma2,
+                            1.f + F::div_const(2.f * gamma * me, mpi, impi) + me * me / (mpi * mpi));
   constexpr float I = (float)(16.0e-9 * 10.75);
-  const float deltahalf = f_log(28.816e-9f * sqrtf(2.33f * 0.498f) / I) + f_log(beta * gamma) - 0.5f;
-  const float dEdx = beta < 1.f
-                         ? (2.f * (xi * invCos * (0.5f * f_log(2.f * me * beta2 * gamma2 * wmax / (I * I)) - beta2 - deltahalf) / beta2))
-                         : 0.f;
-  const float dP = prop_sign * dEdx / beta;
-  par[3] = p / (fmaxf(p + dP, 0.001f) * pt);
-  C[9] += dP * dP / (p2 * pt * pt);  // (3,3)
+  constexpr float I2 = I * I, iI2 = 1.f / I2;
+  // log(28.816e-9 sqrt(2.33 * 0.498) / I), each step rounded to float.
+  constexpr float log_plasma = -1.7122072f;
+  const float deltahalf = log_plasma + m.log(beta * gamma) - 0.5f;
+  const float log_w = m.log(F::div_const(2.f * me * beta2 * gamma2 * wmax, I2, iI2));
+  const float dEdx =
+      beta < 1.f ? (2.f * (F::div(xi * invCos * (0.5f * log_w - beta2 - deltahalf), beta2))) : 0.f;
+  const float dP = F::div(prop_sign * dEdx, beta);
+  par[3] = F::div(p, fmaxf(p + dP, 0.001f) * pt);
+  C[9] += F::div(dP * dP, p2 * pt * pt);  // (3,3)
 }
 
 // Material grid lookup with the reference's bin arithmetic and range guard
@@ -363,21 +430,24 @@ __device__ __forceinline__ void material_lookup(const Material& m, float z, floa
 // Restates propagateHelixToRMPlex (mkFit/PropagationMPlex.cc:408-505).
 // On failure the output is reset to the input (fix-up at :497-504).
 //------------------------------------------------------------------------------
-__device__ __forceinline__ int propagate_to_r(const float (&par)[6], const float (&err)[21], int chg,
-                                              float r, unsigned pflags, const Material& mat,
-                                              bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
+template <class F>
+__device__ __forceinline__ int propagate_to_r_in(F& m, const float (&par)[6], const float (&err)[21],
+                                                 int chg, float r, unsigned pflags,
+                                                 const Material& mat, bool no_mat_eff,
+                                                 float (&opar)[6], float (&oerr)[21]) {
   float J[36];
   float p[6];
-  const int fail = helix_to_r(par, chg, r, pflags & kPfParamB, p, J);
+  float sinT;
+  const int fail = helix_to_r(m, par, chg, r, pflags & kPfParamB, p, J, sinT);
   float C[21];
 #pragma unroll
   for (int i = 0; i < 21; ++i) C[i] = err[i];
   if (pflags & kPfMaterial) {
     float rl = 0.f, xi = 0.f;
     if (!(fail || no_mat_eff)) material_lookup(mat, p[2], r, rl, xi);
-    const float r0 = hipo(par[0], par[1]);
+    const float r0 = F::sqrt(par[0] * par[0] + par[1] * par[1]);
     const float sign = (r > r0 ? 1.f : -1.f);
-    material_effects(rl, xi, sign, true, C, p);
+    material_effects(m, rl, xi, sign, true, sinT, 1.f, C, p);
   }
   p[4] = squash_phi(p[4]);
   float Co[21];
@@ -398,20 +468,23 @@ __device__ __forceinline__ int propagate_to_r(const float (&par)[6], const float
 
 // Propagation to plane z. Restates propagateHelixToZMPlex
 // (mkFit/PropagationMPlex.cc:510-601); this path has no fail flag.
-__device__ __forceinline__ void propagate_to_z(const float (&par)[6], const float (&err)[21], int chg,
-                                               float z, unsigned pflags, const Material& mat,
-                                               bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
+template <class F>
+__device__ __forceinline__ void propagate_to_z_in(F& m, const float (&par)[6], const float (&err)[21],
+                                                  int chg, float z, unsigned pflags,
+                                                  const Material& mat, bool no_mat_eff,
+                                                  float (&opar)[6], float (&oerr)[21]) {
   float J[36];
   float p[6];
-  helix_to_z(par, chg, z, pflags & kPfParamB, p, J);
+  float sinT, cosT;
+  helix_to_z(m, par, chg, z, pflags & kPfParamB, p, J, sinT, cosT);
   float C[21];
 #pragma unroll
   for (int i = 0; i < 21; ++i) C[i] = err[i];
   if (pflags & kPfMaterial) {
     float rl = 0.f, xi = 0.f;
-    if (!no_mat_eff) material_lookup(mat, z, hypot_f(p[0], p[1]), rl, xi);
+    if (!no_mat_eff) material_lookup(mat, z, m.hypot(p[0], p[1]), rl, xi);
     const float sign = (fabsf(z) > fabsf(par[2]) ? 1.f : -1.f);
-    material_effects(rl, xi, sign, false, C, p);
+    material_effects(m, rl, xi, sign, false, sinT, cosT, C, p);
   }
   p[4] = squash_phi(p[4]);
   similarity_endcap(J, C, oerr);
@@ -419,13 +492,90 @@ __device__ __forceinline__ void propagate_to_z(const float (&par)[6], const floa
   for (int i = 0; i < 6; ++i) opar[i] = p[i];
 }
 
+// The steps repeated with ExactMath where FlatMath's operands left their
+// range (rare: a track at the beam line, 1/pT near zero, an overflow). Not
+// inlined, on copies, so the usual path keeps its arrays in registers.
+struct StateCopy {
+  float par[6], err[21];
+};
+static __device__ __noinline__ int propagate_exact(StateCopy* s, bool to_r, int chg, float at,
+                                            unsigned pflags, Material mat, bool no_mat_eff) {
+  ExactMath m;
+  float par[6], err[21];
+  int fail = 0;
+  if (to_r)
+    fail = propagate_to_r_in(m, s->par, s->err, chg, at, pflags, mat, no_mat_eff, par, err);
+  else
+    propagate_to_z_in(m, s->par, s->err, chg, at, pflags, mat, no_mat_eff, par, err);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) s->par[i] = par[i];
+#pragma unroll
+  for (int i = 0; i < 21; ++i) s->err[i] = err[i];
+  return fail;
+}
+
+__device__ __forceinline__ int propagate_again(const float (&par)[6], const float (&err)[21], bool to_r,
+                                               int chg, float at, unsigned pflags, const Material& mat,
+                                               bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
+  StateCopy s;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) s.par[i] = par[i];
+#pragma unroll
+  for (int i = 0; i < 21; ++i) s.err[i] = err[i];
+  const int fail = propagate_exact(&s, to_r, chg, at, pflags, mat, no_mat_eff);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) opar[i] = s.par[i];
+#pragma unroll
+  for (int i = 0; i < 21; ++i) oerr[i] = s.err[i];
+  return fail;
+}
+
+// With ExactMath, and (the *_flat forms) with FlatMath. The fit uses the
+// flat ones. The finding keeps the plain ones: its decisions rest on results
+// pinned bit for bit, and the compiler contracts the flat form's products
+// and sums into other FMAs.
+__device__ __forceinline__ int propagate_to_r(const float (&par)[6], const float (&err)[21], int chg,
+                                              float r, unsigned pflags, const Material& mat,
+                                              bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
+  ExactMath m;
+  return propagate_to_r_in(m, par, err, chg, r, pflags, mat, no_mat_eff, opar, oerr);
+}
+
+__device__ __forceinline__ void propagate_to_z(const float (&par)[6], const float (&err)[21], int chg,
+                                               float z, unsigned pflags, const Material& mat,
+                                               bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
+  ExactMath m;
+  propagate_to_z_in(m, par, err, chg, z, pflags, mat, no_mat_eff, opar, oerr);
+}
+
+__device__ __forceinline__ int propagate_to_r_flat(const float (&par)[6], const float (&err)[21],
+                                                   int chg, float r, unsigned pflags,
+                                                   const Material& mat, bool no_mat_eff,
+                                                   float (&opar)[6], float (&oerr)[21]) {
+  FlatMath m;
+  int fail = propagate_to_r_in(m, par, err, chg, r, pflags, mat, no_mat_eff, opar, oerr);
+  if (!m.ok())
+    fail = propagate_again(par, err, true, chg, r, pflags, mat, no_mat_eff, opar, oerr);
+  return fail;
+}
+
+__device__ __forceinline__ void propagate_to_z_flat(const float (&par)[6], const float (&err)[21],
+                                                    int chg, float z, unsigned pflags,
+                                                    const Material& mat, bool no_mat_eff,
+                                                    float (&opar)[6], float (&oerr)[21]) {
+  FlatMath m;
+  propagate_to_z_in(m, par, err, chg, z, pflags, mat, no_mat_eff, opar, oerr);
+  if (!m.ok()) propagate_again(par, err, false, chg, z, pflags, mat, no_mat_eff, opar, oerr);
+}
+
 //------------------------------------------------------------------------------
 // 2x2 symmetric inverse with the determinant formed in double precision
 // (CramerInverterSym<T,2,N>, Matriplex/MatriplexSym.h:422-445).
 //------------------------------------------------------------------------------
-__device__ __forceinline__ void invert_sym2(float& a0, float& a1, float& a2) {
+template <class F>
+__device__ __forceinline__ void invert_sym2(F& m, float& a0, float& a1, float& a2) {
   const double det = (double)a0 * a2 - (double)a1 * a1;
-  const float s = (float)(1.0 / det);
+  const float s = m.inv_det(det);
   const float tmp = s * a2;
   a1 *= -s;
   a2 = s * a0;
@@ -437,13 +587,13 @@ __device__ __forceinline__ void invert_sym2(float& a0, float& a1, float& a2) {
 // cylinder, chi2 and/or update. Restates kalmanOperation
 // (mkFit/KalmanUtilsMPlex.cc:548-681). do_update: write (opar, oerr).
 //------------------------------------------------------------------------------
-template <bool kChi2, bool kUpdate>
-__device__ __forceinline__ float kalman_barrel(const float (&par)[6], const float (&err)[21],
-                                               const float (&mpos)[3], const float (&merr)[6],
-                                               float (&opar)[6], float (&oerr)[21]) {
-  const float r = hypot_f(mpos[0], mpos[1]);
-  const float r00 = -(mpos[1] + par[1]) / (2 * r);
-  const float r01 = (mpos[0] + par[0]) / (2 * r);
+template <bool kChi2, bool kUpdate, class F>
+__device__ __forceinline__ float kalman_barrel_in(F& m, const float (&par)[6], const float (&err)[21],
+                                                  const float (&mpos)[3], const float (&merr)[6],
+                                                  float (&opar)[6], float (&oerr)[21]) {
+  const float r = m.hypot(mpos[0], mpos[1]);
+  const float r00 = F::div(-(mpos[1] + par[1]), 2 * r);
+  const float r01 = F::div(mpos[0] + par[0], 2 * r);
 
   const float res0 = mpos[0] - par[0], res1 = mpos[1] - par[1], res2 = mpos[2] - par[2];
   // Covariance sum in global position coordinates (upper-left 3x3).
@@ -460,7 +610,7 @@ __device__ __forceinline__ float kalman_barrel(const float (&par)[6], const floa
   float s1 = g3 * r00 + g4 * r01;
   float s2 = g5;
   (void)t2;
-  invert_sym2(s0, s1, s2);
+  invert_sym2(m, s0, s1, s2);
 
   float chi2 = 0.f;
   if (kChi2) chi2 = s0 * loc0 * loc0 + s2 * loc1 * loc1 + 2 * (s1 * loc1 * loc0);
@@ -504,13 +654,13 @@ __device__ __forceinline__ float kalman_barrel(const float (&par)[6], const floa
 // Endcap Kalman operation: xy residual, 6x2 gain. Restates
 // kalmanOperationEndcap (mkFit/KalmanUtilsMPlex.cc:774-888).
 //------------------------------------------------------------------------------
-template <bool kChi2, bool kUpdate>
-__device__ __forceinline__ float kalman_endcap(const float (&par)[6], const float (&err)[21],
-                                               const float (&mpos)[3], const float (&merr)[6],
-                                               float (&opar)[6], float (&oerr)[21]) {
+template <bool kChi2, bool kUpdate, class F>
+__device__ __forceinline__ float kalman_endcap_in(F& m, const float (&par)[6], const float (&err)[21],
+                                                  const float (&mpos)[3], const float (&merr)[6],
+                                                  float (&opar)[6], float (&oerr)[21]) {
   const float res0 = mpos[0] - par[0], res1 = mpos[1] - par[1];
   float s0 = err[0] + merr[0], s1 = err[1] + merr[1], s2 = err[2] + merr[2];
-  invert_sym2(s0, s1, s2);
+  invert_sym2(m, s0, s1, s2);
   float chi2 = 0.f;
   if (kChi2) chi2 = s0 * res0 * res0 + s2 * res1 * res1 + 2 * (s1 * res1 * res0);
   if (kUpdate) {
@@ -529,6 +679,64 @@ __device__ __forceinline__ float kalman_endcap(const float (&par)[6], const floa
     khc_endcap(K, err, KHC);
 #pragma unroll
     for (int i = 0; i < 21; ++i) oerr[i] = err[i] - KHC[i];
+  }
+  return chi2;
+}
+
+template <bool kChi2, bool kUpdate>
+__device__ __forceinline__ float kalman_barrel(const float (&par)[6], const float (&err)[21],
+                                               const float (&mpos)[3], const float (&merr)[6],
+                                               float (&opar)[6], float (&oerr)[21]) {
+  ExactMath m;
+  return kalman_barrel_in<kChi2, kUpdate>(m, par, err, mpos, merr, opar, oerr);
+}
+template <bool kChi2, bool kUpdate>
+__device__ __forceinline__ float kalman_endcap(const float (&par)[6], const float (&err)[21],
+                                               const float (&mpos)[3], const float (&merr)[6],
+                                               float (&opar)[6], float (&oerr)[21]) {
+  ExactMath m;
+  return kalman_endcap_in<kChi2, kUpdate>(m, par, err, mpos, merr, opar, oerr);
+}
+
+// The update with FlatMath, repeated with ExactMath where its operands left
+// their range (see propagate_exact).
+struct HitCopy {
+  float pos[3], err[6];
+};
+template <bool kChi2>
+__device__ __noinline__ float update_exact(StateCopy* s, HitCopy h, bool barrel) {
+  ExactMath m;
+  StateCopy o;
+  const float chi2 = barrel
+                         ? kalman_barrel_in<kChi2, true>(m, s->par, s->err, h.pos, h.err, o.par, o.err)
+                         : kalman_endcap_in<kChi2, true>(m, s->par, s->err, h.pos, h.err, o.par, o.err);
+  *s = o;
+  return chi2;
+}
+
+template <bool kChi2, bool kBarrel>
+__device__ __forceinline__ float update_flat(const float (&par)[6], const float (&err)[21],
+                                             const float (&mpos)[3], const float (&merr)[6],
+                                             float (&opar)[6], float (&oerr)[21]) {
+  FlatMath m;
+  float chi2 = kBarrel ? kalman_barrel_in<kChi2, true>(m, par, err, mpos, merr, opar, oerr)
+                       : kalman_endcap_in<kChi2, true>(m, par, err, mpos, merr, opar, oerr);
+  if (!m.ok()) {
+    StateCopy s;
+    HitCopy h;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) s.par[i] = par[i];
+#pragma unroll
+    for (int i = 0; i < 21; ++i) s.err[i] = err[i];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) h.pos[i] = mpos[i];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) h.err[i] = merr[i];
+    chi2 = update_exact<kChi2>(&s, h, kBarrel);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) opar[i] = s.par[i];
+#pragma unroll
+    for (int i = 0; i < 21; ++i) oerr[i] = s.err[i];
   }
   return chi2;
 }

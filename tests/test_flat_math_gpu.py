@@ -1,0 +1,97 @@
+"""The branch-free arithmetic of the Kalman step (csrc/flat_math.cuh) against
+the plain one on the device: the quotient, reciprocal and root bit for bit
+(every mantissa for the one-operand ones), the double-based functions up to
+the values within ~1e-16 of a rounding boundary, and the operands that send a
+step back to the plain form."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+RCP, DIV, SQRT, SIN, COS, LOG, HYPOT, INV_DET = range(8)
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("flat") / "libflat.so")
+    subprocess.check_call([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode",
+                           "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared",
+                           "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+                           os.path.join(HERE, "flat_math_check.cu"), "-o", out])
+    L = ctypes.CDLL(out)
+    p = ctypes.c_void_p
+    L.flat_math_check.argtypes = [ctypes.c_int, ctypes.c_longlong, p, p, p]
+    L.flat_math_seen.argtypes = [ctypes.c_int, p, ctypes.c_int, p]
+    return L
+
+
+def check(lib, what, n, a=None, b=None):
+    import torch
+    counts = torch.zeros(3, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.flat_math_check(what, n, None if a is None else a.data_ptr(),
+                               None if b is None else b.data_ptr(), counts.data_ptr()) == 0
+    c = counts.cpu().tolist()
+    assert c[2] == 0, "operands outside the safe range"
+    return c[0], c[1]
+
+
+def operands(n, seed, lo, hi, signed=True):
+    """Sizes log-uniform in [lo, hi]."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    u = torch.rand(n, generator=g, device="cuda", dtype=torch.float64)
+    v = torch.exp(np.log(lo) + u * (np.log(hi) - np.log(lo))).float()
+    if signed:
+        v = torch.where(torch.rand(n, generator=g, device="cuda") < 0.5, -v, v)
+    return v
+
+
+@pytest.mark.parametrize("what", [RCP, SQRT])
+def test_every_mantissa(lib, what):
+    # 2^24 consecutive floats from 1: all mantissas in two exponents. The
+    # reciprocal's last step is exact but for a mantissa of all ones, where
+    # 1 / b lies next to a rounding boundary: at most one value per exponent.
+    bad, ulps = check(lib, what, 1 << 24)
+    assert bad <= (2 if what == RCP else 0) and ulps <= 1
+
+
+def test_quotients(lib):
+    n = 1 << 26
+    bad, ulps = check(lib, DIV, n, operands(n, 1, 1e-6, 1e6), operands(n, 2, 1e-6, 1e6))
+    assert bad <= 2 and ulps <= 1
+
+
+@pytest.mark.parametrize("what,lo,hi,signed", [(SIN, 1e-3, 6.4, True), (COS, 1e-3, 6.4, True),
+                                               (SIN, 10.0, 250.0, True), (LOG, 1e-20, 1e20, False),
+                                               (LOG, 0.9, 1.1, False)])
+def test_functions(lib, what, lo, hi, signed):
+    # Two doubles within d = 1e-15 of each other (relative) round to different
+    # floats when a boundary lies between them: about 2 d / 2^-23 of the values.
+    n = 1 << 24
+    bad, ulps = check(lib, what, n, operands(n, 3, lo, hi, signed))
+    assert bad <= 4 and ulps <= 1
+
+
+@pytest.mark.parametrize("what", [HYPOT, INV_DET])
+def test_two_operand_functions(lib, what):
+    n = 1 << 24
+    bad, ulps = check(lib, what, n, operands(n, 5, 1e-2, 1e2, what == HYPOT),
+                      operands(n, 6, 1e-2, 1e2, what == HYPOT))
+    assert bad <= 4 and ulps <= 1
+
+
+def test_operands_outside_the_range(lib):
+    import torch
+    v = torch.tensor([0.0, -0.0, 1.0, -1.0, 1e-7, 1e7, 5e5, 2e-6, float("inf"), -float("inf"),
+                      float("nan"), 1e-40], device="cuda")
+    for wide, exp in ((0, [0, 0, 1, 1, 0, 0, 1, 1, 0, 0, 0, 0]),
+                      (1, [0, 0, 1, 0, 1, 1, 1, 1, 0, 0, 0, 0])):
+        ok = torch.zeros(len(v), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        assert lib.flat_math_seen(len(v), v.data_ptr(), wide, ok.data_ptr()) == 0
+        assert ok.cpu().tolist() == exp
