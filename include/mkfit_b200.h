@@ -422,7 +422,9 @@ int mkfg_find_upload(mkfg_context* ctx, const mkfg_event* ev);
 int mkfg_find_upload_batch(mkfg_context* ctx, const mkfg_event* evs, int32_t n_events);
 int mkfg_find_run(mkfg_context* ctx);
 /* The same sequence captured once per upload into a CUDA graph and
- * replayed (one graph launch per call). No reference counterpart. */
+ * replayed (one graph launch per call). Uploads of up to 7168 seeds run
+ * through the fused form (mkfg_find_run_fused) instead, which is faster
+ * there; so does mkfg_find_event. No reference counterpart. */
 int mkfg_find_run_graph(mkfg_context* ctx);
 /* The plain run with a CUDA event after every launch: kernel_ms[7]
  * receives the device time of each kernel class summed over the layer

@@ -9,9 +9,9 @@
 //                 handling, hole records (one thread per active candidate)
 //   3. chi2     : propagate to each selected hit, chi2, strip checks,
 //                 hit records (one thread per (cand, hit) pair)
-//   4. clone    : per-seed ranking of the records (warp top-M selection),
+//   4. clone    : per-seed ranking of the records (by counting),
 //                 overlap hits, extras, best short candidate, new
-//                 candidates (one warp per seed) -- CandCloner::ProcessSeedRange
+//                 candidates (8 lanes per seed) -- CandCloner::ProcessSeedRange
 //   5. update   : UpdateWithLastHit for the listed candidates that took a hit
 //                 (barrel and endcap candidates listed apart)
 // then one merge launch (MergeCandsAndBestShortOne) and one export launch.
@@ -2115,6 +2115,8 @@ static int enqueue_fused(Finder* f, cudaStream_t st, int w) {
   const int grid_c = (S * kSlots + kBlock - 1) / kBlock;
   k_reset<<<std::max(grid_c, (n_work + kBlock - 1) / kBlock), kBlock, 0, st>>>(f->ev, n_work);
   MKFG_CUDA_TRY(cudaMemsetAsync(f->ev.pair_count, 0, 4 * (size_t)(f->host_cfg.max_steps + 2), st));
+  MKFG_CUDA_TRY(cudaMemsetAsync(f->ev.step_count, 0,
+                                4 * (size_t)kCntN * (f->host_cfg.max_steps + 2), st));
   switch (w) {
     case 4: return launch_fused<4>(f, st);
     case 8: return launch_fused<8>(f, st);
@@ -2122,6 +2124,18 @@ static int enqueue_fused(Finder* f, cudaStream_t st, int w) {
     default: return set_error(MKFG_ERR_BAD_INPUT, "seeds_per_block must be 4, 8 or 16 (got %d)", w);
   }
 }
+
+// Seeds per block with which a run of S seeds goes through the fused form
+// instead of the launch sequence, 0 for the sequence. A sequence of 211
+// launches costs their latency whatever the size (1.45 ms for one event of
+// 120 seeds as a graph, 1.88 ms launch by launch), and the fused form's
+// blocks run through all steps on their own: while they fit the chip at
+// once it takes 0.78 (120 seeds), 0.75 (800) and 0.87 ms (1600) with 8 seeds
+// per block, as against 0.85 with 16 per block there, which are the faster
+// ones beyond (0.95 against 1.39 ms at 3000 seeds, the graph 1.72; 1.93 at
+// 8000, the graph 2.09). The lines: where the two widths cross, and a wave of the
+// 128-thread blocks (three per SM) before the graph is the faster one.
+static int fused_width(int S) { return S <= 1536 ? 8 : S <= 7168 ? 16 : 0; }
 
 // The plain sequence with an event after every launch: device time per
 // kernel class (0 reset, 1 activate, 2 propagate, 3 chi2, 4 clone,
@@ -2190,6 +2204,7 @@ static int run_plain(mkfg_context* ctx, Finder* f) {
 static int run_graph(mkfg_context* ctx, Finder* f) {
   if (f->n_seeds == 0) return MKFG_OK;
   cudaStream_t st = ctx->stream;
+  if (const int w = fused_width(f->n_seeds)) return enqueue_fused(f, st, w);
   // The launches take the device view by value: a graph captured with
   // another one is stale.
   if (f->graph && std::memcmp(&f->graph_ev, &f->ev, sizeof(EventDev)) != 0) f->drop_graph();
@@ -3261,7 +3276,13 @@ extern "C" int mkfg_find_download_best(mkfg_context* ctx, int n_seeds, mkfg_find
 extern "C" int mkfg_find_event(mkfg_context* ctx, const mkfg_event* ev, mkfg_find_out* out) {
   int rc;
   if ((rc = mkfg_find_upload(ctx, ev))) return rc;
-  if ((rc = mkfg_find_run(ctx))) return rc;
+  Finder* f = finder_of(ctx);
+  const int w = fused_width(f->n_seeds);
+  if (w && f->n_seeds > 0) {
+    if ((rc = enqueue_fused(f, ctx->stream, w))) return rc;
+  } else if ((rc = mkfg_find_run(ctx))) {
+    return rc;
+  }
   return mkfg_find_download(ctx, ev->n_seeds, out);
 }
 

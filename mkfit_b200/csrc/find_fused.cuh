@@ -10,8 +10,15 @@
 // they stay in L1/L2 between phases).
 //
 // The per-candidate and per-seed work is the code the plain kernels call
-// (find_steps.cuh), so results are the plain form's; a chunk stops stepping
-// once none of its seeds can change any more.
+// (find_steps.cuh), so results are the plain form's (a hit's chi2 may differ
+// in its last bit, one in 1e5, where the compiler contracted another FMA); a
+// chunk stops stepping once none of its seeds can change any more.
+//
+// Bound by latency: a step is the chain of its four phases in one block
+// (18.5 us per step for 120 seeds, 8 per block: 0.78 ms per run). With a
+// warp per seed in the clone phase 1.18 ms; with the branch-free arithmetic
+// (flat_math.cuh) 0.58, but other FMA contractions, whose rounding turned
+// near-ties of the ranking in one small event out of ten.
 #pragma once
 
 #include "find_steps.cuh"
@@ -31,6 +38,7 @@ struct FusedShared {
   unsigned short pairs[T * kMaxXHits];
   CloneScratch scratch[W];
   int n_pairs;
+  int pairs_end[2];   // of them in barrel and endcap layers
 };
 
 template <int W>
@@ -54,7 +62,7 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
   const int* lb = E.layer_begin + ev * E.lb_stride;
   const int n_local = min(W, E.n_seeds - s0);
 
-  if (tid == 0) S.n_pairs = 0;
+  if (tid == 0) S.n_pairs = S.pairs_end[0] = S.pairs_end[1] = 0;
   __syncthreads();
 
   for (int step = 1; step <= C.max_steps; ++step) {
@@ -72,9 +80,18 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
     const bool active = in_range && layer >= 0 && state == kFinding && c < ncand &&
                         activate_cand(E, B, s, slot, layer, C.looper_stop != 0, par, err, chg);
     const unsigned act = __ballot_sync(0xffffffffu, active) & grp;
+    int* cnt = E.step_count + step * kCntN;
+    const bool barrel = layer >= 0 && C.layer[layer].is_barrel;
     {
       const unsigned all = __ballot_sync(0xffffffffu, active);
-      if (lane == 0 && all) atomicAdd(&E.work[step * kWorkN + 0], __popc(all));
+      const unsigned nb = __popc(__ballot_sync(0xffffffffu, active && barrel));
+      const unsigned nf = __popc(__ballot_sync(0xffffffffu, c == 0 && act != 0));
+      if (lane == 0 && all) {
+        atomicAdd(&E.work[step * kWorkN + 0], __popc(all));
+        if (nb) atomicAdd(cnt + kCntActBarrel, nb);
+        if (nb < __popc(all)) atomicAdd(cnt + kCntActEndcap, __popc(all) - nb);
+        atomicAdd(cnt + kCntFind, nf);
+      }
     }
     if (in_range && c == 0) {
       if (layer >= 0 && state == kFinding && act == 0) state = kFinished;
@@ -92,6 +109,7 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
 #pragma unroll
       for (int e = 0; e < 21; ++e) S.perr[e * T + tid] = o.perr[e];
       if (o.xs > 0) {
+        atomicAdd(S.pairs_end + !barrel, o.xs);
         const int base = atomicAdd(&S.n_pairs, o.xs);
         for (int h = 0; h < o.xs; ++h) S.pairs[base + h] = (unsigned short)(tid * kMaxXHits + h);
       }
@@ -106,6 +124,8 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
     if (tid == 0 && np) {
       atomicAdd(&E.pair_count[step], np);
       atomicAdd(&E.work[step * kWorkN + 2], np);
+      if (S.pairs_end[0]) atomicAdd(cnt + kCntPairBarrel, S.pairs_end[0]);
+      if (S.pairs_end[1]) atomicAdd(cnt + kCntPairEndcap, S.pairs_end[1]);
     }
     for (int p = tid; p < np; p += T) {
       const int code = S.pairs[p];
@@ -135,7 +155,7 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
     __syncthreads();
 
     //-------------------------------------------------------------- clone
-    if (tid == 0) S.n_pairs = 0;
+    if (tid == 0) S.n_pairs = S.pairs_end[0] = S.pairs_end[1] = 0;
     // The 8 threads of a seed rank its records, then each writes a new
     // candidate and updates it with the hit it took.
     {
@@ -145,6 +165,8 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
       const CloneList l = clone_rank(E, C, on, on ? s : 0, layer, ncand, buf, R, S.scratch[ls], lane);
       if (on && c == 0) {
         atomicAdd(&E.work[step * kWorkN + 3], 1);
+        atomicAdd(&E.work[step * kWorkN + 4], l.n_records);
+        atomicAdd(&E.work[step * kWorkN + 5], l.n);
         E.n_cands[s] = l.n;
         E.cur[s] = buf ^ 1;
       }
@@ -153,6 +175,7 @@ __global__ void __launch_bounds__(W * kSlots) k_find_fused(EventDev E,
         //-------------------------------------------------------------- update
         if (upd) {
           atomicAdd(&E.work[step * kWorkN + 1], 1);
+          atomicAdd(cnt + (barrel ? kCntUpdBarrel : kCntUpdEndcap), 1);
           update_cand_at(E, C, C.layer[layer], lb[layer] + upd - 1, E.cand[buf],
                          s * kSlots + l.parent, E.cand[buf ^ 1], slot);
         }

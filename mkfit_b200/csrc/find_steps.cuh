@@ -1,6 +1,6 @@
 // Per-candidate and per-seed steps of one clone-engine layer iteration.
 // Each function restates the cited reference routine for one candidate
-// (one CUDA thread) or one seed (one warp); the plain form calls them from
+// (one CUDA thread) or one seed (8 lanes); the plain form calls them from
 // separate kernels, the batched persistent form from one kernel.
 #pragma once
 
@@ -390,7 +390,7 @@ __device__ __forceinline__ void prep_cand(const EventDev& E, const FindConfigDev
                                           int slot, const float (&par)[6], const float (&err)[21],
                                           int chg, int* xhit, int xstride, PrepOut& o) {
   if (L.is_barrel)
-    propagate_to_r(par, err, chg, L.propagate_to, C.inter_pflags, C.mat, false, o.ppar, o.perr);
+    propagate_to_r<true>(par, err, chg, L.propagate_to, C.inter_pflags, C.mat, false, o.ppar, o.perr);
   else
     propagate_to_z(par, err, chg, L.propagate_to, C.inter_pflags, C.mat, false, o.ppar, o.perr);
   select_cand<kGenericBins>(E, C, L, layer_bins, hit_base, reg, layer, s, B, slot, o.ppar, o.perr,
@@ -445,8 +445,8 @@ __device__ __forceinline__ bool pair_accept(const EventDev& E, const FindConfigD
   float hpar[6], herr_[21];
   float chi2;
   if (L.is_barrel) {
-    propagate_to_r(ppar, perr, chg, hypot_f(mpos[0], mpos[1]), C.intra_pflags, C.mat, false, hpar,
-                   herr_);
+    propagate_to_r<true>(ppar, perr, chg, hypot_f(mpos[0], mpos[1]), C.intra_pflags, C.mat, false,
+                         hpar, herr_);
     chi2 = kalman_barrel<true, false>(hpar, herr_, mpos, merr, hpar, herr_);
   } else {
     propagate_to_z(ppar, perr, chg, mpos[2], C.intra_pflags, C.mat, false, hpar, herr_);
@@ -508,7 +508,8 @@ __device__ __forceinline__ void update_state(const EventDev& E, const FindConfig
   load_hit(E, g, mpos, merr);
   float ppar[6], perr[21];
   if (L.is_barrel) {
-    propagate_to_r(par, err, chg, hypot_f(mpos[0], mpos[1]), C.inter_pflags, C.mat, false, ppar, perr);
+    propagate_to_r<true>(par, err, chg, hypot_f(mpos[0], mpos[1]), C.inter_pflags, C.mat, false, ppar,
+                         perr);
     kalman_barrel<false, true>(ppar, perr, mpos, merr, par, err);
   } else {
     propagate_to_z(par, err, chg, mpos[2], C.inter_pflags, C.mat, false, ppar, perr);

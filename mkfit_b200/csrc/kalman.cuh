@@ -171,7 +171,10 @@ __device__ __forceinline__ void curvature(F& m, int chg, bool param_b, float z, 
   kinv = F::rcp(k);
 }
 
-template <class F>
+// kPinned: one product and difference with their own roundings, for the
+// finding (left to the compiler, the launch sequence's and the fused form's
+// (candidate, hit) kernels were contracted differently there, and only there).
+template <bool kPinned = false, class F>
 __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, float r, bool param_b,
                                           float (&out)[6], float (&J)[36], float& sinT) {
 #pragma unroll
@@ -286,7 +289,8 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
   J[2 * 6 + 0] = k * cosT * dadx * pt * isinT;
   J[2 * 6 + 1] = k * cosT * dady * pt * isinT;
   J[2 * 6 + 2] = 1.f;
-  J[2 * 6 + 3] = k * cosT * (ipt * dadipt - alpha) * pt * pt * isinT;
+  const float dalpha = kPinned ? __fsub_rn(__fmul_rn(ipt, dadipt), alpha) : ipt * dadipt - alpha;
+  J[2 * 6 + 3] = k * cosT * dalpha * pt * pt * isinT;
   J[2 * 6 + 4] = k * dadphi * cosT * pt * isinT;
   J[2 * 6 + 5] = -k * alpha * pt * isinT * isinT;
 
@@ -430,7 +434,7 @@ __device__ __forceinline__ void material_lookup(const Material& m, float z, floa
 // Restates propagateHelixToRMPlex (mkFit/PropagationMPlex.cc:408-505).
 // On failure the output is reset to the input (fix-up at :497-504).
 //------------------------------------------------------------------------------
-template <class F>
+template <bool kPinned = false, class F>
 __device__ __forceinline__ int propagate_to_r_in(F& m, const float (&par)[6], const float (&err)[21],
                                                  int chg, float r, unsigned pflags,
                                                  const Material& mat, bool no_mat_eff,
@@ -438,7 +442,7 @@ __device__ __forceinline__ int propagate_to_r_in(F& m, const float (&par)[6], co
   float J[36];
   float p[6];
   float sinT;
-  const int fail = helix_to_r(m, par, chg, r, pflags & kPfParamB, p, J, sinT);
+  const int fail = helix_to_r<kPinned>(m, par, chg, r, pflags & kPfParamB, p, J, sinT);
   float C[21];
 #pragma unroll
   for (int i = 0; i < 21; ++i) C[i] = err[i];
@@ -534,11 +538,12 @@ __device__ __forceinline__ int propagate_again(const float (&par)[6], const floa
 // flat ones. The finding keeps the plain ones: its decisions rest on results
 // pinned bit for bit, and the compiler contracts the flat form's products
 // and sums into other FMAs.
+template <bool kPinned = false>
 __device__ __forceinline__ int propagate_to_r(const float (&par)[6], const float (&err)[21], int chg,
                                               float r, unsigned pflags, const Material& mat,
                                               bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
   ExactMath m;
-  return propagate_to_r_in(m, par, err, chg, r, pflags, mat, no_mat_eff, opar, oerr);
+  return propagate_to_r_in<kPinned>(m, par, err, chg, r, pflags, mat, no_mat_eff, opar, oerr);
 }
 
 __device__ __forceinline__ void propagate_to_z(const float (&par)[6], const float (&err)[21], int chg,

@@ -354,6 +354,49 @@ def test_fused_equals_plain(gpu_ctx, w):
         assert wf[k] == wp[k], (k, wf[k], wp[k])
 
 
+@pytest.mark.parametrize("sizes,it", [((1,), 0), ((1536,), 0), ((1200, 337), 3), ((40, 90), 7),
+                                      ((900, 4, 600), 6), ((7168,), 0), ((4200, 2969), 1)],
+                         ids=lambda v: "-".join(map(str, v)) if isinstance(v, tuple) else f"it{v}")
+def test_small_uploads_equal_plain(gpu_ctx, sizes, it):
+    """run_graph and find_event on both sides of the seed counts at which
+    they turn from the fused form (8, then 16 seeds per block) to the launch
+    sequence: the candidates, work counts and step counts of the plain run,
+    for iterations with other plans, windows and (7) host-sorted seeds."""
+    cfg = FindConfig(iteration=it, max_cands=M)
+    fnd = Finder(gpu_ctx, cfg)
+    events = []
+    for i, n in enumerate(sizes):
+        ev = synth.gen_cms_event(int(1.02 * n) + 40, seed=500 + i, noise_frac=0.05)
+        d = dict(ev.__dict__)
+        d.update({k: np.ascontiguousarray(d[k][:, :n]) for k in ("seed_par", "seed_err")})
+        d.update({k: np.ascontiguousarray(d[k][:n]) for k in (
+            "seed_chg", "seed_nhits", "seed_hit_layer", "seed_hit_index", "seed_mc")})
+        events.append(synth.CmsEvent(**d))
+        assert events[-1].n_seeds == n
+    total = fnd.upload_batch(events)
+    fnd.run()
+    want, w_work, w_steps = fnd.download(total), fnd.work(), fnd.step_profile(timed=False)
+    fnd.run_graph()
+    got, g_work, g_steps = fnd.download(total), fnd.work(), fnd.step_profile(timed=False)
+    runs = [(got, want)]
+    if len(events) == 1:
+        runs.append((fnd.find_event(events[0]), got))
+    for a, b in runs:
+        for k in a:
+            if k in ("chi2", "score"):
+                # A hit's chi2 may differ in its last bit (another FMA
+                # contraction in one of the kernels, one hit in 1e5); the sum
+                # of at most 64 hits then differs by at most 64 * 2^-24.
+                np.testing.assert_allclose(a[k], b[k], rtol=64 * 2.0 ** -24,
+                                           atol=64 * 2.0 ** -24 * 64, err_msg=k)
+            else:
+                np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+    for k in ("active_cands", "hit_pairs", "updates", "seed_steps"):
+        assert g_work[k] == w_work[k], k
+    for k in fnd.STEP_COUNTS:
+        np.testing.assert_array_equal(g_steps[k], w_steps[k], err_msg=k)
+
+
 def test_fused_autotune_and_repeat(gpu_ctx):
     events = [synth.gen_cms_event(n, seed=300 + n) for n in (800, 300)]
     fnd = Finder(gpu_ctx, FindConfig(max_cands=M))
