@@ -15,8 +15,17 @@
 namespace mkfg {
 namespace adj {
 
-AD_FN float ad_sqrt(float x) { return sqrtf(x); }
-AD_FN double ad_sqrt(double x) { return sqrt(x); }
+// Quotient and root, and the operands whose size they need in a safe range:
+// here the plain forms, for any material argument; adjoint.cu adds the
+// branch-free ones for its own.
+template <typename T, typename MatT>
+AD_FN T ad_div(const MatT&, T a, T b) { return a / b; }
+template <typename T, typename MatT>
+AD_FN void ad_see(const MatT&, T) {}
+template <typename MatT>
+AD_FN float ad_sqrt(const MatT&, float x) { return sqrtf(x); }
+template <typename MatT>
+AD_FN double ad_sqrt(const MatT&, double x) { return sqrt(x); }
 AD_FN float ad_log(float x) { return logf(x); }
 AD_FN double ad_log(double x) { return log(x); }
 AD_FN float ad_sin(float x) { return sinf(x); }

@@ -19,6 +19,8 @@ emitter writes
 
 Both are C++ templates over the arithmetic type: float in the CUDA kernels,
 double on the host for checking the derivation against finite differences.
+Divisions and roots are calls that take the material argument `mat`, whose
+type chooses their form (adjoint_step.cuh).
 
     python gen_adjoint.py      # rewrites generated_adjoint.cuh
 """
@@ -395,6 +397,7 @@ class Emitter:
     def __init__(self, g):
         self.g = g
         self.names = {}
+        self.seen = set()
 
     def ref(self, n):
         if n.op == "const":
@@ -452,9 +455,9 @@ class Emitter:
                 "add": lambda: "%s + %s" % (A[0], A[1]),
                 "sub": lambda: "%s - %s" % (A[0], A[1]),
                 "mul": lambda: "%s * %s" % (A[0], A[1]),
-                "div": lambda: "%s / %s" % (A[0], A[1]),
+                "div": lambda: "ad_div(mat, %s, %s)" % (A[0], A[1]),
                 "neg": lambda: "-%s" % A[0],
-                "sqrt": lambda: "ad_sqrt(%s)" % A[0],
+                "sqrt": lambda: "ad_sqrt(mat, %s)" % A[0],
                 "log": lambda: "ad_log(%s)" % A[0],
                 "sin": lambda: "ad_sin(%s)" % A[0],
                 "cos": lambda: "ad_cos(%s)" % A[0],
@@ -462,13 +465,19 @@ class Emitter:
                 "max": lambda: "ad_max(%s, %s)" % (A[0], A[1]),
                 "select": lambda: "%s ? %s : %s" % (A[0], A[1], A[2]),
             }[op]()
+            # Operands whose size the division, root or logarithm (whose
+            # adjoint divides by it) needs in range: shown to `mat` once each.
+            watched = {"div": 1, "sqrt": 0, "log": 0}.get(op)
+            if watched is not None and n.args[watched].op != "const" and \
+                    n.args[watched].id not in self.seen:
+                self.seen.add(n.args[watched].id)
+                lines.append("  ad_see(mat, %s);" % A[watched])
             lines.append("  const T %s = %s;" % (v, expr))
         return order
 
     def reverse(self, order, outputs, out_bar_names, inputs, lines):
         gname = {}
         node = self.g.nodes
-
         def acc(n, expr):
             if n.op in ("const", "in_nd") or n.is_bool or n.op.startswith("out"):
                 return
@@ -504,13 +513,13 @@ class Emitter:
                     acc(A[1], "%s * %s" % (g, R[0]))
             elif op == "div":
                 q = "q%d" % i
-                lines.append("  const T %s = %s / %s;" % (q, g, R[1]))
+                lines.append("  const T %s = ad_div(mat, %s, %s);" % (q, g, R[1]))
                 acc(A[0], q)
                 acc(A[1], "-%s * %s" % (q, self.names[i]))
             elif op == "sqrt":
-                acc(A[0], "T(0.5) * %s / %s" % (g, self.names[i]))
+                acc(A[0], "ad_div(mat, T(0.5) * %s, %s)" % (g, self.names[i]))
             elif op == "log":
-                acc(A[0], "%s / %s" % (g, R[0]))
+                acc(A[0], "ad_div(mat, %s, %s)" % (g, R[0]))
             elif op == "sin":
                 acc(A[0], "%s * ad_cos(%s)" % (g, R[0]))
             elif op == "cos":
