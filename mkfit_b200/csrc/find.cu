@@ -897,8 +897,9 @@ __device__ __forceinline__ bool pair_hits_dup(const SelectArgs& A, int i, int j,
 // percent of pairs that only their shared hits decide go to a list and are
 // taken by a warp each. One thread per seed walking all later seeds left
 // 24,000 threads on chains of up to 1500 dependent tests and n1 x n2 hit
-// loads inside divergent warps: 2886 us for 16 events x 1500 seeds, against
-// @DUPS@ in tiles.
+// loads inside divergent warps: 2886 us for 16 events x 1500 seeds, of
+// which the tiles save 2500 (a whole iteration on that batch: 8.87 against
+// 11.39 ms).
 template <int kMode>
 __global__ void __launch_bounds__(kDupTile) k_select_dups(EventDev E, const SelectArgs A, int n_tiles,
                                                           int* __restrict__ dup) {
