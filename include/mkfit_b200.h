@@ -442,10 +442,8 @@ int mkfg_find_step_profile(mkfg_context* ctx, float* launch_ms, int32_t* counts)
 /* Fused form of the same run: one launch in which every thread block carries
  * seeds_per_block consecutive seeds (4, 8 or 16; 0 = the value chosen by
  * mkfg_find_autotune, 16 before any tuning) through all layer steps and the
- * final merge, with the step scratch in shared memory. Same candidates and
- * hit lists as mkfg_find_run; candidate states agree to FP32 rounding (the
- * shared step code may be contracted into FMAs differently). No reference
- * counterpart. */
+ * final merge, with the step scratch in shared memory. Same results as
+ * mkfg_find_run, bit for bit. No reference counterpart. */
 int mkfg_find_run_fused(mkfg_context* ctx, int32_t seeds_per_block);
 /* Times mkfg_find_run_fused on the uploaded events for every supported
  * seeds_per_block, keeps the fastest for later calls with 0, and returns it

@@ -21,6 +21,11 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-Xptxas", "-warn-spills"]
+# The Kalman step's sources: products and sums rounded as they are written
+# (the FMAs are explicit), so that every kernel built from the step -- the fit,
+# the operator calls, each form of the finding -- gives the same bits. Left to
+# the compiler, a kernel's surroundings decide what it contracts.
+SRC_FLAGS = {"find.cu": ["-fmad=false"], "fit.cu": ["-fmad=false"], "operators.cu": ["-fmad=false"]}
 
 
 def _newer(dst, srcs):
@@ -53,7 +58,7 @@ def build(verbose=False, extra_flags=(), out_dir=None):
         obj = os.path.join(obj_dir, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
         if _newer(obj, [src] + headers):
-            cmd = [NVCC] + ARCH + FLAGS + list(extra_flags) + ["-c", src, "-o", obj]
+            cmd = [NVCC] + ARCH + FLAGS + SRC_FLAGS.get(os.path.basename(src), []) + list(extra_flags) + ["-c", src, "-o", obj]
             if verbose:
                 print(" ".join(cmd))
             subprocess.check_call(cmd)

@@ -201,7 +201,7 @@ __device__ __forceinline__ int hot_layer(int v) { return v >> 24; }
 __device__ __forceinline__ float score_calc(int nfound, int ntail, int nover, int nmiss, float chi2,
                                             float pt, bool in_find) {
   const float maxBonus = 8.0f;
-  float bonus = 0.2f * nfound + 4.0f;
+  float bonus = fmaf(0.2f, nfound, 4.0f);
   float penalty = 8.0f;
   const float tailPenalty = 3.0f;
   const float overlapBonus = 0.0f;

@@ -10,15 +10,15 @@
 // they stay in L1/L2 between phases).
 //
 // The per-candidate and per-seed work is the code the plain kernels call
-// (find_steps.cuh), so results are the plain form's (a hit's chi2 may differ
-// in its last bit, one in 1e5, where the compiler contracted another FMA); a
-// chunk stops stepping once none of its seeds can change any more.
+// (find_steps.cuh), with every rounding written out, so results are the plain
+// form's bit for bit; a chunk stops stepping once none of its seeds can change
+// any more.
 //
 // Bound by latency: a step is the chain of its four phases in one block
 // (18.5 us per step for 120 seeds, 8 per block: 0.78 ms per run). With a
 // warp per seed in the clone phase 1.18 ms; with the branch-free arithmetic
-// (flat_math.cuh) 0.58, but other FMA contractions, whose rounding turned
-// near-ties of the ranking in one small event out of ten.
+// (flat_math.cuh) 0.58, measured when the compiler chose the FMAs and other
+// ones turned near-ties of the ranking in one small event out of ten.
 #pragma once
 
 #include "find_steps.cuh"

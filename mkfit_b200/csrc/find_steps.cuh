@@ -56,12 +56,12 @@ __device__ __forceinline__ void dynamic_windows(const LayerDev& L, float invpt, 
                                                 float& max_dphi) {
   float max_invpt = invpt;
   if (invpt > 10.0) max_invpt = 10.0f;
-  const float this_dq = L.c_dq_0 * max_invpt + L.c_dq_1 * theta + L.c_dq_2;
+  const float this_dq = fmaf(L.c_dq_1, theta, L.c_dq_0 * max_invpt) + L.c_dq_2;
   if (L.c_dq_sf * this_dq > 0.f) {
     min_dq = L.c_dq_sf * this_dq;
     max_dq = 2.0f * min_dq;
   }
-  const float this_dphi = L.c_dp_0 * max_invpt + L.c_dp_1 * theta + L.c_dp_2;
+  const float this_dphi = fmaf(L.c_dp_1, theta, L.c_dp_0 * max_invpt) + L.c_dp_2;
   if (L.c_dp_sf * this_dphi > min_dphi) {
     min_dphi = L.c_dp_sf * this_dphi;
     max_dphi = 2.0f * min_dphi;
@@ -75,7 +75,7 @@ __device__ __forceinline__ float dynamic_chi2_cut(const LayerDev& L, float chi2_
   const float theta = fabsf(par[5] - kPIOver2);
   float max_invpt = invpt;
   if (invpt > 10.0) max_invpt = 10.0f;
-  const float this_c2 = L.c_c2_0 * max_invpt + L.c_c2_1 * theta + L.c_c2_2;
+  const float this_c2 = fmaf(L.c_c2_1, theta, L.c_c2_0 * max_invpt) + L.c_c2_2;
   if (L.c_c2_sf * this_c2 > chi2_min) return L.c_c2_sf * this_c2;
   return chi2_min;
 }
@@ -113,7 +113,8 @@ __device__ __forceinline__ int select_hits(const EventDev& E, const LayerDev& L,
   const float x = par[0], y = par[1];
   const float r2 = x * x + y * y;
   const float dphidx = -y / r2, dphidy = x / r2;
-  const float dphi2 = dphidx * dphidx * err[0] + dphidy * dphidy * err[2] + 2 * dphidx * dphidy * err[1];
+  const float dphi2 = fmaf(2 * dphidx * dphidy, err[1],
+                           fmaf(dphidx * dphidx, err[0], dphidy * dphidy * err[2]));
   const float phi = f_atan2(y, x);
   float dphi = fmaxf(3.f * sqrtf(fabsf(dphi2)), min_dphi);
   float q, dq;
@@ -121,7 +122,7 @@ __device__ __forceinline__ int select_hits(const EventDev& E, const LayerDev& L,
     const float z = par[2];
     dq = fabsf(3.f * sqrtf(err[5]));
     const float edgeCorr = fabsf(0.5f * (L.rout - L.rin) / f_tan(par[5]));
-    const float d = sqrtf(dq * dq + edgeCorr * edgeCorr);
+    const float d = sqrtf(fmaf(dq, dq, edgeCorr * edgeCorr));
     if (z > L.zmax + d || z < L.zmin - d)
       wsr = kWsrOutside;
     else if (z < L.zmax - d && z > L.zmin + d)
@@ -131,9 +132,9 @@ __device__ __forceinline__ int select_hits(const EventDev& E, const LayerDev& L,
     q = z;
   } else {
     const float r = sqrtf(r2);
-    dq = 3.f * sqrtf(fabsf(x * x * err[0] + y * y * err[2] + 2 * x * y * err[1]) / r2);
+    dq = 3.f * sqrtf(fabsf(fmaf(2 * x * y, err[1], fmaf(x * x, err[0], y * y * err[2]))) / r2);
     const float edgeCorr = fabsf(0.5f * (L.zmax - L.zmin) * f_tan(par[5]));
-    const float d = sqrtf(dq * dq + edgeCorr * edgeCorr);
+    const float d = sqrtf(fmaf(dq, dq, edgeCorr * edgeCorr));
     if (r > L.rout + d || r < L.rin - d) {
       wsr = kWsrOutside;
     } else if (r < L.rout - d && r > L.rin + d) {
@@ -203,8 +204,9 @@ __device__ __forceinline__ bool strip_q_compatible(bool barrel, const float (&pe
   const float hitT2 = merr[0] + merr[2];
   const float hitT2inv = 1.f / hitT2;
   const float proj0 = merr[0] * hitT2inv, proj1 = merr[1] * hitT2inv, proj2 = merr[2] * hitT2inv;
-  const float qErr = sqrtf(fabsf(perr[0] * proj0 + 2.f * perr[1] * proj1 + perr[2] * proj2));
-  const float resProj = sqrtf(res0 * proj0 * res0 + 2.f * res1 * proj1 * res0 + res1 * proj2 * res1);
+  const float qErr = sqrtf(fabsf(fmaf(perr[2], proj2, fmaf(perr[0], proj0, 2.f * perr[1] * proj1))));
+  const float resProj =
+      sqrtf(fmaf(res1 * proj2, res1, fmaf(res0 * proj0, res0, 2.f * res1 * proj1 * res0)));
   return sqrtf(hitT2 * 3.f) + fmaxf(3.f * qErr, 0.5f) > resProj;
 }
 
@@ -218,12 +220,12 @@ __device__ __forceinline__ bool strip_charge_ok(bool barrel, unsigned pcm, const
     const float hitT2 = merr[0] + merr[2];
     const float hitT2inv = 1.f / hitT2;
     const float proj0 = merr[0] * hitT2inv, proj1 = merr[1] * hitT2inv, proj2 = merr[2] * hitT2inv;
-    const bool detXY_OK = fabsf(proj0 * proj2 - proj1 * proj1) < 0.1f;
+    const bool detXY_OK = fabsf(fmaf(proj0, proj2, -(proj1 * proj1))) < 0.1f;
     const float cosP = f_cos(ppar[4]);
     const float sinP = f_sin(ppar[4]);
     const float sinT = fabsf(f_sin(ppar[5]));
-    qSF = detXY_OK ? sinT * sqrtf(fabsf(1.f + cosP * cosP * proj0 + sinP * sinP * proj2 -
-                                        2.f * cosP * sinP * proj1))
+    qSF = detXY_OK ? sinT * sqrtf(fabsf(fmaf(-2.f * cosP * sinP, proj1,
+                                             fmaf(sinP * sinP, proj2, fmaf(cosP * cosP, proj0, 1.f)))))
                    : 1.f;
   } else {
     qSF = fabsf(f_cos(ppar[5]));
@@ -353,7 +355,7 @@ __device__ __forceinline__ bool cand_is_active(const EventDev& E, const CandSoA&
   const float pt = fabsf(1.f / ipt);
   if (looper_stop && pt < 1.2f) {  // IT_FwdSearch only
     const float dphi = fabsf(f_atan2(y, x) - phi);
-    if (x * x + y * y > 625.f && dphi > 1.371f && dphi < 4.512f) {
+    if (fmaf(x, x, y * y) > 625.f && dphi > 1.371f && dphi < 4.512f) {
       B.last[slot] = arena_append(E, s, -2, layer, 0.f, last);
       B.nmiss[slot] += 1;
       return false;
@@ -390,7 +392,7 @@ __device__ __forceinline__ void prep_cand(const EventDev& E, const FindConfigDev
                                           int slot, const float (&par)[6], const float (&err)[21],
                                           int chg, int* xhit, int xstride, PrepOut& o) {
   if (L.is_barrel)
-    propagate_to_r<true>(par, err, chg, L.propagate_to, C.inter_pflags, C.mat, false, o.ppar, o.perr);
+    propagate_to_r<false>(par, err, chg, L.propagate_to, C.inter_pflags, C.mat, false, o.ppar, o.perr);
   else
     propagate_to_z(par, err, chg, L.propagate_to, C.inter_pflags, C.mat, false, o.ppar, o.perr);
   select_cand<kGenericBins>(E, C, L, layer_bins, hit_base, reg, layer, s, B, slot, o.ppar, o.perr,
@@ -445,7 +447,7 @@ __device__ __forceinline__ bool pair_accept(const EventDev& E, const FindConfigD
   float hpar[6], herr_[21];
   float chi2;
   if (L.is_barrel) {
-    propagate_to_r<true>(ppar, perr, chg, hypot_f(mpos[0], mpos[1]), C.intra_pflags, C.mat, false,
+    propagate_to_r<false>(ppar, perr, chg, hypot_f(mpos[0], mpos[1]), C.intra_pflags, C.mat, false,
                          hpar, herr_);
     chi2 = kalman_barrel<true, false>(hpar, herr_, mpos, merr, hpar, herr_);
   } else {
@@ -508,7 +510,7 @@ __device__ __forceinline__ void update_state(const EventDev& E, const FindConfig
   load_hit(E, g, mpos, merr);
   float ppar[6], perr[21];
   if (L.is_barrel) {
-    propagate_to_r<true>(par, err, chg, hypot_f(mpos[0], mpos[1]), C.inter_pflags, C.mat, false, ppar,
+    propagate_to_r<false>(par, err, chg, hypot_f(mpos[0], mpos[1]), C.inter_pflags, C.mat, false, ppar,
                          perr);
     kalman_barrel<false, true>(ppar, perr, mpos, merr, par, err);
   } else {

@@ -72,6 +72,22 @@ class TMat(Mat):
         return self.base.entry(j, i)
 
 
+def fma_sum(terms):
+    """The sum of the terms, in order, as explicit FMAs: one rounding order
+    whatever the compiler does around it. Each product is fused onto the sum
+    before it, the first one onto the rounded second."""
+    if len(terms) > 1 and "*" in terms[0] and "*" in terms[1]:
+        terms = [terms[1], terms[0]] + terms[2:]
+    acc = terms[0]
+    for t in terms[1:]:
+        if "*" in t:
+            a, b = t.split(" * ")
+            acc = f"fmaf({a}, {b}, {acc})"
+        else:
+            acc = f"{acc} + {t}"
+    return acc
+
+
 def product(a, b, out_name, out_sym=False, out_pattern=None):
     """Emit out = a * b. Returns (lines, flops, out Mat)."""
     assert a.cols == b.rows
@@ -114,7 +130,7 @@ def product(a, b, out_name, out_sym=False, out_pattern=None):
             else:
                 f = max(0, n_copy - 1)
             flops += f
-            lines.append(f"  {out_name}[{idx}] = {' + '.join(terms)};")
+            lines.append(f"  {out_name}[{idx}] = {fma_sum(terms)};")
     return lines, flops, Mat(out_name, rows, cols, pat, out_sym)
 
 

@@ -6,6 +6,12 @@
 // 6x6 covariance as 21 floats (packed lower triangle, same element order as
 // the reference's MatriplexSym), 6x6 Jacobians as 36-float arrays whose
 // known-zero entries are folded away by the generated products.
+//
+// Every sum of products says which product is fused (fmaf) and which is
+// rounded, and the fit's, the operator calls' and the finding's sources are
+// compiled without the compiler's own contraction (build.py), so all their
+// kernels give the same bits. The choice is the one the compiler had made in
+// the finding's launch sequence.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -100,13 +106,13 @@ __device__ __forceinline__ float f_atan2(float y, float x) {
 }
 
 // sqrt(x*x + y*y) in float, as the reference's hipo() (Matrix.h:38).
-__device__ __forceinline__ float hipo(float x, float y) { return sqrtf(x * x + y * y); }
+__device__ __forceinline__ float hipo(float x, float y) { return sqrtf(fmaf(x, x, y * y)); }
 
 // std::hypot(float, float) as evaluated by glibc: the sum of squares is
 // formed in double precision and the root is rounded once to float.
 __device__ __forceinline__ float hypot_f(float x, float y) {
   const double dx = x, dy = y;
-  return (float)sqrt(dx * dx + dy * dy);
+  return (float)sqrt(fma(dx, dx, dy * dy));
 }
 
 // The plain form of the step's arithmetic (flat_math.cuh).
@@ -127,14 +133,14 @@ struct ExactMath {
 
 // Magnetic field model (Config.h:434-437).
 __device__ __forceinline__ float bfield_zr(float z, float r) {
-  return (kMagB0 * z * z + kMagB1 * z + kMagC1) * (kMagA * r * r + 1.f);
+  return (fmaf(kMagB0 * z, z, kMagB1 * z) + kMagC1) * fmaf(kMagA * r, r, 1.f);
 }
 
 // Fourth-order sin/cos polynomial of the reference (Matrix.h:48-56).
 __device__ __forceinline__ void sincos4(float x, float& s, float& c) {
   const float x2 = x * x;
-  c = 1.f - 0.5f * x2 + 0.04166667f * x2 * x2;
-  s = x - 0.16666667f * x * x2;
+  c = fmaf(0.04166667f * x2, x2, fmaf(-0.5f, x2, 1.f));
+  s = fmaf(-0.16666667f * x, x2, x);
 }
 
 // phi into [-pi, pi) (squashPhiMPlex, mkFit/PropagationMPlex.h:8-15).
@@ -171,17 +177,17 @@ __device__ __forceinline__ void curvature(F& m, int chg, bool param_b, float z, 
   kinv = F::rcp(k);
 }
 
-// kPinned: one product and difference with their own roundings, for the
-// finding (left to the compiler, the launch sequence's and the fused form's
-// (candidate, hit) kernels were contracted differently there, and only there).
-template <bool kPinned = false, class F>
+// kResidual: the 1/pT derivative of z takes ipt * dadipt - alpha, which nearly
+// cancels, from the exact product (the fits) or from the rounded one (the
+// finding and its operator calls).
+template <bool kResidual = true, class F>
 __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, float r, bool param_b,
                                           float (&out)[6], float (&J)[36], float& sinT) {
 #pragma unroll
   for (int i = 0; i < 36; ++i) J[i] = 0.f;
   int fail = 0;
 
-  float r02 = in[0] * in[0] + in[1] * in[1];
+  float r02 = fmaf(in[0], in[0], in[1] * in[1]);
   m.see(r02);
   float r0 = F::sqrt(r02);
   float k, kinv;
@@ -206,11 +212,11 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
 #pragma unroll
   for (int it = 0; it < kNiter; ++it) {
     if (it > 0) {
-      r02 = ox * ox + oy * oy;
+      r02 = fmaf(ox, ox, oy * oy);
       m.see(r02);
       r0 = F::sqrt(r02);
     }
-    const float dot = pxin * ox + pyin * oy;
+    const float dot = fmaf(pxin, ox, pyin * oy);
     m.see(dot);
     const float oodotp = F::div(r0 * pt, dot);
     if (oodotp > 5.0f || oodotp < 0) {
@@ -222,8 +228,12 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
     D += id;
 
     sincos4(id * ipt * kinv * 0.5f, sinah, cosah);
-    cosa = 1.f - 2.f * sinah * sinah;
+    cosa = fmaf(-2.f * sinah, sinah, 1.f);
     sina = 2.f * sinah * cosah;
+    // The direction after the step.
+    const float pxca = pxin * cosa, pxsa = pxin * sina;
+    const float pyca = pyin * cosa, pysa = pyin * sina;
+    const float pxnew = pxca - pysa, pynew = pyca + pxsa;
 
     // Far from the target radius (the first steps) the factor 1 / r0 of
     // every derivative term is 0: FlatMath, whose numbers are finite, skips
@@ -235,44 +245,48 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
       const float dadipt = id * kinv;
       const float dadx = -x * ipt * kinv * oor0;
       const float dady = -y * ipt * kinv * oor0;
-      const float pxca = pxin * cosa;
-      const float pxsa = pxin * sina;
-      const float pyca = pyin * cosa;
-      const float pysa = pyin * sina;
       float tmp = k * dadx;
-      dDdx -= (x * (1.f + tmp * (pxca - pysa)) + y * tmp * (pyca + pxsa)) * oor0;
+      dDdx = fmaf(-fmaf(y * tmp, pynew, x * fmaf(tmp, pxnew, 1.f)), oor0, dDdx);
       tmp = k * dady;
-      dDdy -= (x * tmp * (pxca - pysa) + y * (1.f + tmp * (pyca + pxsa))) * oor0;
+      dDdy = fmaf(-fmaf(x * tmp, pxnew, y * fmaf(tmp, pynew, 1.f)), oor0, dDdy);
       tmp = dadipt * ipt;
-      dDdipt -= k * (x * (pxca * tmp - pysa * tmp - pyca - pxsa + pyin) +
-                     y * (pyca * tmp + pxsa * tmp - pysa + pxca - pxin)) * pt * oor0;
-      dDdphi += k * (x * (pysa - pxin + pxca) - y * (pxsa - pyin + pyca)) * oor0;
+      const float a = fmaf(-pxin, sina, fmaf(-pyin, cosa, fmaf(pxca, tmp, -(pysa * tmp)))) + pyin;
+      const float b = fmaf(pxin, cosa, fmaf(-pyin, sina, fmaf(pyca, tmp, pxsa * tmp))) - pxin;
+      dDdipt = fmaf(-(k * fmaf(x, a, y * b) * pt), oor0, dDdipt);
+      const float u = fmaf(pxin, cosa, fmaf(pyin, sina, -pxin));
+      const float v = fmaf(pyin, cosa, fmaf(pxin, sina, -pyin));
+      dDdphi = fmaf(k * fmaf(x, u, -(y * v)), oor0, dDdphi);
     }
 
-    ox = ox + 2.f * k * sinah * (pxin * cosah - pyin * sinah);
-    oy = oy + 2.f * k * sinah * (pyin * cosah + pxin * sinah);
-    const float pxinold = pxin;
-    pxin = pxin * cosa - pyin * sina;
-    pyin = pyin * cosa + pxinold * sina;
+    ox = fmaf(2.f * k * sinah, fmaf(pxin, cosah, -(pyin * sinah)), ox);
+    oy = fmaf(2.f * k * sinah, fmaf(pxin, sinah, pyin * cosah), oy);
+    pxin = pxnew;
+    pyin = pynew;
   }
 
   const float alpha = D * ipt * kinv;
   const float dadx = dDdx * ipt * kinv;
   const float dady = dDdy * ipt * kinv;
-  const float dadipt = (ipt * dDdipt + D) * kinv;
+  const float dadipt = fmaf(ipt, dDdipt, D) * kinv;
   const float dadphi = dDdphi * ipt * kinv;
 
   sincos4(alpha, sina, cosa);
 
-  J[0 * 6 + 0] = 1.f + k * dadx * (cosPorT * cosa - sinPorT * sina) * pt;
-  J[0 * 6 + 1] = k * dady * (cosPorT * cosa - sinPorT * sina) * pt;
-  J[0 * 6 + 3] = k * (cosPorT * (ipt * dadipt * cosa - sina) + sinPorT * ((1.f - cosa) - ipt * dadipt * sina)) * pt * pt;
-  J[0 * 6 + 4] = k * (cosPorT * dadphi * cosa - sinPorT * dadphi * sina - sinPorT * sina + cosPorT * cosa - cosPorT) * pt;
+  // Sine and cosine of the direction's azimuth at the end, and the 1/pT terms.
+  const float ca = fmaf(cosPorT, cosa, -(sinPorT * sina));
+  const float sa = fmaf(cosPorT, sina, sinPorT * cosa);
+  const float w = ipt * dadipt;
+  const float wc = fmaf(w, cosa, -sina), ws = fmaf(w, sina, -(1.f - cosa));
 
-  J[1 * 6 + 0] = k * dadx * (sinPorT * cosa + cosPorT * sina) * pt;
-  J[1 * 6 + 1] = 1.f + k * dady * (sinPorT * cosa + cosPorT * sina) * pt;
-  J[1 * 6 + 3] = k * (sinPorT * (ipt * dadipt * cosa - sina) + cosPorT * (ipt * dadipt * sina - (1.f - cosa))) * pt * pt;
-  J[1 * 6 + 4] = k * (sinPorT * dadphi * cosa + cosPorT * dadphi * sina + sinPorT * cosa + cosPorT * sina - sinPorT) * pt;
+  J[0 * 6 + 0] = fmaf(k * dadx * ca, pt, 1.f);
+  J[0 * 6 + 1] = k * dady * ca * pt;
+  J[0 * 6 + 3] = k * fmaf(cosPorT, wc, sinPorT * -ws) * pt * pt;
+  J[0 * 6 + 4] = k * (fmaf(cosPorT, cosa, fmaf(cosPorT * dadphi, cosa, -(sinPorT * dadphi * sina)) - sinPorT * sina) - cosPorT) * pt;
+
+  J[1 * 6 + 0] = k * dadx * sa * pt;
+  J[1 * 6 + 1] = fmaf(k * dady * sa, pt, 1.f);
+  J[1 * 6 + 3] = k * fmaf(sinPorT, wc, cosPorT * ws) * pt * pt;
+  J[1 * 6 + 4] = k * (fmaf(cosPorT, sina, fmaf(sinPorT, cosa, fmaf(sinPorT * dadphi, cosa, cosPorT * dadphi * sina))) - sinPorT) * pt;
 
   float cosT;
   m.sincos(theta, &sinT, &cosT);
@@ -281,7 +295,7 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
 
   out[0] = ox;
   out[1] = oy;
-  out[2] = in[2] + k * alpha * cosT * pt * isinT;
+  out[2] = fmaf(k * alpha * cosT * pt, isinT, in[2]);
   out[3] = ipt;
   out[4] = in[4] + alpha;
   out[5] = theta;
@@ -289,7 +303,7 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
   J[2 * 6 + 0] = k * cosT * dadx * pt * isinT;
   J[2 * 6 + 1] = k * cosT * dady * pt * isinT;
   J[2 * 6 + 2] = 1.f;
-  const float dalpha = kPinned ? __fsub_rn(__fmul_rn(ipt, dadipt), alpha) : ipt * dadipt - alpha;
+  const float dalpha = kResidual ? fmaf(ipt, dadipt, -alpha) : w - alpha;
   J[2 * 6 + 3] = k * cosT * dalpha * pt * pt * isinT;
   J[2 * 6 + 4] = k * dadphi * cosT * pt * isinT;
   J[2 * 6 + 5] = -k * alpha * pt * isinT * isinT;
@@ -299,7 +313,7 @@ __device__ __forceinline__ int helix_to_r(F& m, const float (&in)[6], int chg, f
   J[4 * 6 + 0] = dadx;
   J[4 * 6 + 1] = dady;
   J[4 * 6 + 3] = dadipt;
-  J[4 * 6 + 4] = 1.f + dadphi;
+  J[4 * 6 + 4] = fmaf(dDdphi * ipt, kinv, 1.f);
 
   J[5 * 6 + 5] = 1.f;
   return fail;
@@ -340,26 +354,27 @@ __device__ __forceinline__ void helix_to_z(F& m, const float (&in)[6], int chg, 
 
   float sinah, cosah;
   sincos4(alpha * 0.5f, sinah, cosah);
-  const float cosa = 1.f - 2.f * sinah * sinah;
+  const float cosa = fmaf(-2.f * sinah, sinah, 1.f);
   const float sina = 2.f * sinah * cosah;
 
-  out[0] = in[0] + 2.f * k * sinah * (pxin * cosah - pyin * sinah);
-  out[1] = in[1] + 2.f * k * sinah * (pyin * cosah + pxin * sinah);
+  out[0] = fmaf(2.f * k * sinah, fmaf(pxin, cosah, -(pyin * sinah)), in[0]);
+  out[1] = fmaf(2.f * k * sinah, fmaf(pxin, sinah, pyin * cosah), in[1]);
   out[2] = zout;
   out[3] = in[3];
   out[4] = phiin + alpha;
   out[5] = in[5];
 
-  const float pxcaMpysa = pxin * cosa - pyin * sina;
+  const float ac = fmaf(alpha, cosa, -sina), as = fmaf(-alpha, cosah, sinah);
+  const float pxcaMpysa = fmaf(pxin, cosa, -(pyin * sina));
   J[0 * 6 + 2] = -tanT * ipt * pxcaMpysa;
-  J[0 * 6 + 3] = k * pt * pt * (cosP * (alpha * cosa - sina) + sinP * 2.f * sinah * (sinah - alpha * cosah));
-  J[0 * 6 + 4] = -2 * k * pt * sinah * (sinP * cosah + cosP * sinah);
+  J[0 * 6 + 3] = k * pt * pt * fmaf(sinP * 2.f * sinah, as, cosP * ac);
+  J[0 * 6 + 4] = -2 * k * pt * sinah * fmaf(cosP, sinah, sinP * cosah);
   J[0 * 6 + 5] = deltaZ * ipt * pxcaMpysa * icos2T;
 
-  const float pycaPpxsa = pyin * cosa + pxin * sina;
+  const float pycaPpxsa = fmaf(pxin, sina, pyin * cosa);
   J[1 * 6 + 2] = -tanT * ipt * pycaPpxsa;
-  J[1 * 6 + 3] = k * pt * pt * (sinP * (alpha * cosa - sina) - cosP * 2.f * sinah * (sinah - alpha * cosah));
-  J[1 * 6 + 4] = 2 * k * pt * sinah * (cosP * cosah - sinP * sinah);
+  J[1 * 6 + 3] = k * pt * pt * fmaf(sinP, ac, -(cosP * 2.f * sinah * as));
+  J[1 * 6 + 4] = 2 * k * pt * sinah * fmaf(cosP, cosah, -(sinP * sinah));
   J[1 * 6 + 5] = deltaZ * ipt * pycaPpxsa * icos2T;
 
   J[4 * 6 + 2] = -ipt * tanT * kinv;
@@ -392,10 +407,9 @@ __device__ __forceinline__ void material_effects(F& m, float radL, float xi, flo
   const float invCos = is_barrel ? F::div(p, pt) : F::rcp(fabsf(cosT));
   radL = radL * invCos;
   if (radL < 1e-13f) return;
-  const float thetaMSC = F::div(0.0136f * (1.f + 0.038f * m.log(radL)), beta * p);
-  const float thetaMSC2 = thetaMSC * thetaMSC * radL;
-  C[14] += thetaMSC2;  // (4,4)
-  C[20] += thetaMSC2;  // (5,5)
+  const float thetaMSC = F::div(0.0136f * fmaf(0.038f, m.log(radL), 1.f), beta * p);
+  C[14] = fmaf(thetaMSC * thetaMSC, radL, C[14]);  // (4,4)
+  C[20] = fmaf(thetaMSC * thetaMSC, radL, C[20]);  // (5,5)
   constexpr float impi2 = 1.f / mpi2, impi = 1.f / mpi;
   const float gamma2 = F::div_const(p2 + mpi2, mpi2, impi2);
   const float gamma = F::sqrt(gamma2);
@@ -409,7 +423,7 @@ __device__ __forceinline__ void material_effects(F& m, float radL, float xi, flo
   const float deltahalf = log_plasma + m.log(beta * gamma) - 0.5f;
   const float log_w = m.log(F::div_const(2.f * me * beta2 * gamma2 * wmax, I2, iI2));
   const float dEdx =
-      beta < 1.f ? (2.f * (F::div(xi * invCos * (0.5f * log_w - beta2 - deltahalf), beta2))) : 0.f;
+      beta < 1.f ? (2.f * (F::div(xi * invCos * (fmaf(0.5f, log_w, -beta2) - deltahalf), beta2))) : 0.f;
   const float dP = F::div(prop_sign * dEdx, beta);
   par[3] = F::div(p, fmaxf(p + dP, 0.001f) * pt);
   C[9] += F::div(dP * dP, p2 * pt * pt);  // (3,3)
@@ -434,7 +448,7 @@ __device__ __forceinline__ void material_lookup(const Material& m, float z, floa
 // Restates propagateHelixToRMPlex (mkFit/PropagationMPlex.cc:408-505).
 // On failure the output is reset to the input (fix-up at :497-504).
 //------------------------------------------------------------------------------
-template <bool kPinned = false, class F>
+template <bool kResidual = true, class F>
 __device__ __forceinline__ int propagate_to_r_in(F& m, const float (&par)[6], const float (&err)[21],
                                                  int chg, float r, unsigned pflags,
                                                  const Material& mat, bool no_mat_eff,
@@ -442,14 +456,14 @@ __device__ __forceinline__ int propagate_to_r_in(F& m, const float (&par)[6], co
   float J[36];
   float p[6];
   float sinT;
-  const int fail = helix_to_r<kPinned>(m, par, chg, r, pflags & kPfParamB, p, J, sinT);
+  const int fail = helix_to_r<kResidual>(m, par, chg, r, pflags & kPfParamB, p, J, sinT);
   float C[21];
 #pragma unroll
   for (int i = 0; i < 21; ++i) C[i] = err[i];
   if (pflags & kPfMaterial) {
     float rl = 0.f, xi = 0.f;
     if (!(fail || no_mat_eff)) material_lookup(mat, p[2], r, rl, xi);
-    const float r0 = F::sqrt(par[0] * par[0] + par[1] * par[1]);
+    const float r0 = F::sqrt(fmaf(par[0], par[0], par[1] * par[1]));
     const float sign = (r > r0 ? 1.f : -1.f);
     material_effects(m, rl, xi, sign, true, sinT, 1.f, C, p);
   }
@@ -535,15 +549,15 @@ __device__ __forceinline__ int propagate_again(const float (&par)[6], const floa
 }
 
 // With ExactMath, and (the *_flat forms) with FlatMath. The fit uses the
-// flat ones. The finding keeps the plain ones: its decisions rest on results
-// pinned bit for bit, and the compiler contracts the flat form's products
-// and sums into other FMAs.
-template <bool kPinned = false>
+// flat ones, the finding the plain ones: with FlatMath its propagation and
+// update were 6 and 13% faster, but its chi2 6% slower, and the double
+// functions' rare other rounding would turn near-ties of its decisions.
+template <bool kResidual = true>
 __device__ __forceinline__ int propagate_to_r(const float (&par)[6], const float (&err)[21], int chg,
                                               float r, unsigned pflags, const Material& mat,
                                               bool no_mat_eff, float (&opar)[6], float (&oerr)[21]) {
   ExactMath m;
-  return propagate_to_r_in<kPinned>(m, par, err, chg, r, pflags, mat, no_mat_eff, opar, oerr);
+  return propagate_to_r_in<kResidual>(m, par, err, chg, r, pflags, mat, no_mat_eff, opar, oerr);
 }
 
 __device__ __forceinline__ void propagate_to_z(const float (&par)[6], const float (&err)[21], int chg,
@@ -579,7 +593,7 @@ __device__ __forceinline__ void propagate_to_z_flat(const float (&par)[6], const
 //------------------------------------------------------------------------------
 template <class F>
 __device__ __forceinline__ void invert_sym2(F& m, float& a0, float& a1, float& a2) {
-  const double det = (double)a0 * a2 - (double)a1 * a1;
+  const double det = fma((double)a0, (double)a2, -((double)a1 * a1));
   const float s = m.inv_det(det);
   const float tmp = s * a2;
   a1 *= -s;
@@ -606,19 +620,17 @@ __device__ __forceinline__ float kalman_barrel_in(F& m, const float (&par)[6], c
   const float g3 = err[3] + merr[3], g4 = err[4] + merr[4], g5 = err[5] + merr[5];
 
   // Local residual and its covariance (ProjectResErr / ProjectResErrTransp).
-  const float loc0 = r00 * res0 + r01 * res1;
+  const float loc0 = fmaf(r00, res0, r01 * res1);
   const float loc1 = res2;
-  const float t0 = r00 * g0 + r01 * g1;
-  const float t1 = r00 * g1 + r01 * g2;
-  const float t2 = r00 * g3 + r01 * g4;
-  float s0 = t0 * r00 + t1 * r01;
-  float s1 = g3 * r00 + g4 * r01;
+  const float t0 = fmaf(r00, g0, r01 * g1);
+  const float t1 = fmaf(r00, g1, r01 * g2);
+  float s0 = fmaf(t0, r00, t1 * r01);
+  float s1 = fmaf(g3, r00, g4 * r01);
   float s2 = g5;
-  (void)t2;
   invert_sym2(m, s0, s1, s2);
 
   float chi2 = 0.f;
-  if (kChi2) chi2 = s0 * loc0 * loc0 + s2 * loc1 * loc1 + 2 * (s1 * loc1 * loc0);
+  if (kChi2) chi2 = fmaf(2.f, s1 * loc1 * loc0, fmaf(s0 * loc0, loc0, s2 * loc1 * loc1));
 
   if (kUpdate) {
     // H^T G (KalmanHTG): 3x2 live block.
@@ -630,11 +642,11 @@ __device__ __forceinline__ float kalman_barrel_in(F& m, const float (&par)[6], c
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       const float ci0 = err[sidx(i, 0)], ci1 = err[sidx(i, 1)], ci2 = err[sidx(i, 2)];
-      K[2 * i + 0] = ci0 * h00 + ci1 * h10 + ci2 * h20;
-      K[2 * i + 1] = ci0 * h01 + ci1 * h11 + ci2 * h21;
+      K[2 * i + 0] = fmaf(ci2, h20, fmaf(ci0, h00, ci1 * h10));
+      K[2 * i + 1] = fmaf(ci2, h21, fmaf(ci0, h01, ci1 * h11));
     }
 #pragma unroll
-    for (int i = 0; i < 6; ++i) opar[i] = par[i] + K[2 * i] * loc0 + K[2 * i + 1] * loc1;
+    for (int i = 0; i < 6; ++i) opar[i] = fmaf(K[2 * i + 1], loc1, fmaf(K[2 * i], loc0, par[i]));
     opar[4] = squash_phi(opar[4]);
     // KH (KHMult): rows (K0*r00, K0*r01, K1, 0, 0, 0).
     float KH[36];
@@ -667,18 +679,18 @@ __device__ __forceinline__ float kalman_endcap_in(F& m, const float (&par)[6], c
   float s0 = err[0] + merr[0], s1 = err[1] + merr[1], s2 = err[2] + merr[2];
   invert_sym2(m, s0, s1, s2);
   float chi2 = 0.f;
-  if (kChi2) chi2 = s0 * res0 * res0 + s2 * res1 * res1 + 2 * (s1 * res1 * res0);
+  if (kChi2) chi2 = fmaf(2.f, s1 * res1 * res0, fmaf(s0 * res0, res0, s2 * res1 * res1));
   if (kUpdate) {
     // K = C[:, 0:2] * S^-1 (KalmanGain62).
     float K[12];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       const float ci0 = err[sidx(i, 0)], ci1 = err[sidx(i, 1)];
-      K[2 * i + 0] = ci0 * s0 + ci1 * s1;
-      K[2 * i + 1] = ci0 * s1 + ci1 * s2;
+      K[2 * i + 0] = fmaf(ci0, s0, ci1 * s1);
+      K[2 * i + 1] = fmaf(ci0, s1, ci1 * s2);
     }
 #pragma unroll
-    for (int i = 0; i < 6; ++i) opar[i] = par[i] + K[2 * i] * res0 + K[2 * i + 1] * res1;
+    for (int i = 0; i < 6; ++i) opar[i] = fmaf(K[2 * i + 1], res1, fmaf(K[2 * i], res0, par[i]));
     opar[4] = squash_phi(opar[4]);
     float KHC[21];
     khc_endcap(K, err, KHC);

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kOpBlock) k_op_propagate(const OpArgs A) {
   if (A.endcap)
     propagate_to_z(p, e, A.chg[i], A.target[i], A.pflags, A.mat, false, op, oe);
   else
-    propagate_to_r(p, e, A.chg[i], A.target[i], A.pflags, A.mat, false, op, oe);
+    propagate_to_r<false>(p, e, A.chg[i], A.target[i], A.pflags, A.mat, false, op, oe);
 #pragma unroll
   for (int k = 0; k < 6; ++k) A.out_par[k * A.stride + i] = op[k];
 #pragma unroll
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kOpBlock) k_op_chi2(const OpArgs A) {
     propagate_to_z(p, e, A.chg[i], m[2], A.pflags, A.mat, false, hp, he);
     chi2 = kalman_endcap<true, false>(hp, he, m, v, hp, he);
   } else {
-    propagate_to_r(p, e, A.chg[i], hypot_f(m[0], m[1]), A.pflags, A.mat, false, hp, he);
+    propagate_to_r<false>(p, e, A.chg[i], hypot_f(m[0], m[1]), A.pflags, A.mat, false, hp, he);
     chi2 = kalman_barrel<true, false>(hp, he, m, v, hp, he);
   }
   A.out_chi2[i] = chi2;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kOpBlock) k_op_update(const OpArgs A) {
     propagate_to_z(p, e, chg, m[2], A.pflags, A.mat, false, hp, he);
     kalman_endcap<false, true>(hp, he, m, v, p, e);
   } else {
-    propagate_to_r(p, e, chg, hypot_f(m[0], m[1]), A.pflags, A.mat, false, hp, he);
+    propagate_to_r<false>(p, e, chg, hypot_f(m[0], m[1]), A.pflags, A.mat, false, hp, he);
     kalman_barrel<false, true>(hp, he, m, v, p, e);
   }
   if (p[3] < 0) {
