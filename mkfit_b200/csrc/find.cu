@@ -56,7 +56,8 @@ constexpr int kBlock = 256;
 #define MKFG_ACT_MIN_BLOCKS 8
 #endif
 // The clone kernel, bound by dependent loads: 64 registers at 4 blocks
-// (5.26 ms per 64-event step; 5 blocks 5.79, 6 blocks 7.54: spills).
+// (5.26 ms per 64-event step when measured; 5 blocks 5.79, 6 blocks 7.54:
+// spills).
 #ifndef MKFG_CLONE_MIN_BLOCKS
 #define MKFG_CLONE_MIN_BLOCKS 4
 #endif
@@ -429,9 +430,11 @@ __global__ void __launch_bounds__(kBlock, MKFG_CHI2_MIN_BLOCKS) k_chi2(EventDev 
 // fewer instructions a seed takes the more of them are in flight: a warp
 // per seed issued 970 instructions for work that keeps 8 lanes busy, a
 // thread per seed left 10 warps on an SM (260 us in the busiest step of the
-// 64-event batch). 64-event batch, 42 steps: clone 5.26 against 7.52 ms a
-// warp per seed, with the update at 2.33 against 1.93 (it now gathers the
-// parents' states); 3.9 TB/s of DRAM traffic, 270 instructions per seed.
+// 64-event batch). 64-event batch, 42 steps: clone 5.0 against 7.4 ms a
+// warp per seed, with the update at 2.2 against 1.9 (it now gathers the
+// parents' states). Dense noise (12 records per seed and step, 8 events of
+// 1500 seeds): 0.87 against 1.01 ms; there the ranking takes the records in
+// turn by all 8 lanes (each lane its own candidate's 1.21 ms).
 //------------------------------------------------------------------------------
 // kCount: also count the records present and the new candidates (work
 // counters 4 and 5), for the eager launch sequence.

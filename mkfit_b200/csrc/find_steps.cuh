@@ -636,97 +636,73 @@ __device__ __forceinline__ CloneList clone_rank(const EventDev& E, const FindCon
   const int n_valid = __shfl_sync(kFull, at, kSlots - 1, kSlots);
   at -= __popc(cm);
   const unsigned em0 = (__ballot_sync(kFull, kind != 0) >> g0) & 0xffu;
-  const bool listed = n_valid <= kCloneList;
-  if (listed) {
-    // The first two records' loads go out together (a candidate seldom has
-    // more than a hit or two and the hole).
-    uint32_t m = cm;
-    const int h0 = m ? __ffs(m) - 1 : 0;
-    m &= m - 1;
-    const int h1 = m ? __ffs(m) - 1 : 0;
-    Record r0{0, 0, 0.f, 0.f}, r1{0, 0, 0.f, 0.f};
-    if (cm) r0 = R.rec(c * kRecPerCand + h0);
-    if (m) r1 = R.rec(c * kRecPerCand + h1);
-    if (cm) {
-      X.key[at] = score_key(r0.score);
-      X.id[at] = clone_id(c * kRecPerCand + h0, r0.hit);
-    }
-    if (m) {
-      X.key[at + 1] = score_key(r1.score);
-      X.id[at + 1] = clone_id(c * kRecPerCand + h1, r1.hit);
-      m &= m - 1;
-    }
-    for (int p = at + 2; m; m &= m - 1, ++p) {
-      const int idx = c * kRecPerCand + __ffs(m) - 1;
-      const Record r = R.rec(idx);
-      X.key[p] = score_key(r.score);
-      X.id[p] = clone_id(idx, r.hit);
-    }
-  }
-  __syncwarp();
 
   // Top-num_hits records in (score desc, record index asc) order: the
   // reference's std::sort by score; on exact score ties this order is the
   // stable one. Record p goes to the place given by the count of those
-  // before it.
+  // before it. More records than places are taken in rounds, the best so far
+  // first. The 8 lanes take the records in turn, whosever they are: a seed
+  // in dense noise has one candidate's dozen hits, and one lane would wait
+  // for them one after the other.
   const int num_hits = min(n_valid, M);
   constexpr int kPer = kCloneList / kSlots;
-  int key[kPer], id[kPer], rank[kPer];
+  int base = 0, kept = 0;
+  do {
+    const bool more = base < n_valid;
+    const int n = more ? min(kept + n_valid - base, kCloneList) : 0;
+    if (more) {
+      int p = kept + at - base;
+      for (uint32_t m = cm; m; m &= m - 1, ++p)
+        if (p >= kept && p < n) X.id[p] = c * kRecPerCand + __ffs(m) - 1;
+    }
+    __syncwarp();
+    int key[kPer], id[kPer], rank[kPer];
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int p = c + kSlots * k;
-    rank[k] = kCloneList;
-    if (listed && kSlots * k < n_valid) {
-      const bool in = p < n_valid;
-      key[k] = in ? X.key[p] : kNoKey;
-      id[k] = in ? X.id[p] : 0;
-      int r = 0;
-      for (int j = 0; j < n_valid; ++j) {
+    for (int k = 0; k < kPer; ++k) {
+      const int p = c + kSlots * k;
+      rank[k] = p < n ? 0 : kCloneList;
+      key[k] = kNoKey;
+      id[k] = 0;
+      if (p < n) {
+        id[k] = X.id[p];
+        if (p >= kept) {
+          const Record r = R.rec(id[k]);
+          key[k] = score_key(r.score);
+          id[k] = clone_id(id[k], r.hit);
+        } else {
+          key[k] = X.key[p];
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (c + kSlots * k < n) X.key[c + kSlots * k] = key[k];
+    __syncwarp();
+    if (n <= kSlots) {
+      for (int j = 0; j < n; ++j) {
         const int kj = X.key[j];
-        r += (kj > key[k]) || (kj == key[k] && j < p);
+        rank[0] += (kj > key[0]) || (kj == key[0] && j < c);
       }
-      if (in) rank[k] = r;
-    }
-  }
-  __syncwarp();
+    } else {
+      for (int j = 0; j < n; ++j) {
+        const int kj = X.key[j];
 #pragma unroll
-  for (int k = 0; k < kPer; ++k)
-    if (rank[k] < num_hits) {
-      X.key[rank[k]] = key[k];
-      X.id[rank[k]] = id[k];
-    }
-  if (!listed) {
-    // More records than places: num_hits rounds, each the best of what is
-    // left (lane c looks through candidate c's records).
-    uint32_t left = cm;
-    for (int i = 0; i < num_hits; ++i) {
-      int bk = kNoKey, bi = INT_MAX, bv = 0;
-      for (uint32_t m = left; m; m &= m - 1) {
-        const int idx = c * kRecPerCand + __ffs(m) - 1;
-        const Record r = R.rec(idx);
-        if (score_key(r.score) > bk) {
-          bk = score_key(r.score);
-          bi = idx;
-          bv = clone_id(idx, r.hit);
-        }
+        for (int k = 0; k < kPer; ++k)
+          rank[k] += (kj > key[k]) || (kj == key[k] && j < c + kSlots * k);
       }
-      int wk = bk, wi = bi;
+    }
+    __syncwarp();
 #pragma unroll
-      for (int off = kSlots / 2; off > 0; off >>= 1) {
-        const int ok = __shfl_xor_sync(gmask, wk, off, kSlots);
-        const int oi = __shfl_xor_sync(gmask, wi, off, kSlots);
-        if (ok > wk || (ok == wk && oi < wi)) {
-          wk = ok;
-          wi = oi;
-        }
+    for (int k = 0; k < kPer; ++k)
+      if (rank[k] < num_hits) {
+        X.key[rank[k]] = key[k];
+        X.id[rank[k]] = id[k];
       }
-      if (bi == wi) {
-        X.key[i] = bk;
-        X.id[i] = bv;
-        left &= ~(1u << (bi - c * kRecPerCand));
-      }
+    if (more) {
+      base += n - kept;
+      kept = min(n, num_hits);
     }
-  }
+  } while (__any_sync(kFull, base < n_valid));
   __syncwarp();
 
   // The new candidate list. The best short candidate's score decides

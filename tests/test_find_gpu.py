@@ -860,13 +860,15 @@ def test_update_with_last_hit_worker_matches_reference(gpu_ctx, reflib, layer):
     assert np.percentile(e64g, 99.9) <= 1.5 * np.percentile(e64r, 99.9) + 1e-6
 
 
-def clone_inputs(n_seeds, rng, m=M):
+def clone_inputs(n_seeds, rng, m=M, dense=False):
     """Seeds for the clone worker: 1..m candidates each (random states and
     counters, ~15% held back: 10% as they are, 5% with a stop node), the
     others with 0..10 hit records (distinct hits on two or three modules,
     so overlap pairs form; chi2 under and over the overlap cut; continuous
     scores, so no two records tie) and a hole record (-1, -2 or -3) with
-    probability 0.8; 30% of the seeds hold a best short candidate."""
+    probability 0.8; 30% of the seeds hold a best short candidate. dense:
+    8..16 hit records per candidate (up to 136 per seed) and whole-number
+    scores, so that many tie."""
     from mkfit_b200.finder import CLONE_IN_FIELDS, clone_arrays
     S = n_seeds
     a = clone_arrays(CLONE_IN_FIELDS, S)
@@ -894,7 +896,7 @@ def clone_inputs(n_seeds, rng, m=M):
     for k in range(K):
         if k % 8 >= nc[k // 8] or a["held_back"][k]:
             continue
-        nh = int(rng.integers(0, 11))
+        nh = int(rng.integers(8, 17) if dense else rng.integers(0, 11))
         hits = rng.choice(5000, nh, replace=False)
         mods = rng.choice(rng.integers(100, 110, 3), nh)
         j = 0
@@ -908,6 +910,8 @@ def clone_inputs(n_seeds, rng, m=M):
             a["rec_module"][k, j] = -1
             a["rec_score"][k, j] = rng.uniform(-10, 50)
             j += 1
+        if dense:
+            a["rec_score"][k, :j] = np.round(a["rec_score"][k, :j])
         a["n_rec"][k] = j
     a["bshort_valid"][:] = rng.random(S) < 0.3
     a["bshort_score"][:] = rng.uniform(-10, 50, S)
@@ -1003,13 +1007,15 @@ def restate_clone(inp, s, m, cfg):
     return out, short
 
 
-@pytest.mark.parametrize("m,n_seeds", [(1, 1), (2, 31), (3, 33), (6, 700), (8, 257)])
-def test_clone_worker_matches_restatement(gpu_ctx, m, n_seeds):
+@pytest.mark.parametrize("m,n_seeds,dense", [(1, 1, 0), (2, 31, 0), (3, 33, 0), (6, 700, 0),
+                                             (8, 257, 0), (1, 40, 1), (6, 97, 1), (8, 257, 1)])
+def test_clone_worker_matches_restatement(gpu_ctx, m, n_seeds, dense):
     """The clone step (ranking and writing) against its restatement: the new
     candidates in order, their parents' states bit for bit, and the best
-    short candidate, for every list length."""
+    short candidate, for every list length; dense: lists ranked in up to six
+    rounds, with ties, which keep record order."""
     from mkfit_b200.finder import NO_HIT
-    inp = clone_inputs(n_seeds, np.random.default_rng(100 + m), m)
+    inp = clone_inputs(n_seeds, np.random.default_rng(100 + m), m, dense)
     cfg = FindConfig(max_cands=m, chi2_cut=30.0, zero_c2=True)
     cuts = dict(chi2_cut_overlap=cfg.c.chi2_cut_overlap, pt_cut_overlap=cfg.c.pt_cut_overlap)
     got = Finder(gpu_ctx, cfg).clone_seeds(4, inp)
