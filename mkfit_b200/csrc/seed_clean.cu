@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstring>
 #include <vector>
 
 namespace mkfg {
@@ -62,8 +63,8 @@ struct CleanDev {
   int* ebin;            // [n]
   int* bin_count;       // [n_events][kEtaBins + 1]
   int* order;           // [n] seeds of each event by eta bin
-  int2* pairs;          // [n_events][pair_stride] overlapping (ts, tss), global seed indices
-  int pair_stride;
+  int2* pairs;          // overlapping (ts, tss), global seed indices, by event
+  const long long* pair_begin;  // [n_events + 1] each event's places in pairs
   int* ev_pairs;        // [n_events] pairs of each event
   int* n_pairs;         // all pairs
   int* comp;            // [n] component label: smallest seed of the component
@@ -216,7 +217,8 @@ __global__ void __launch_bounds__(kCleanBlock) k_clean_pairs(CleanDev D, CleanPa
     const int tss = D.order[s0 + k];
     if (tss <= ts || !seeds_overlap(D, P, ts, tss)) continue;
     const int at = atomicAdd(D.ev_pairs + e, 1);
-    if (at < D.pair_stride) D.pairs[(size_t)e * D.pair_stride + at] = make_int2(ts, tss);
+    const long long to = D.pair_begin[e] + at;
+    if (to < D.pair_begin[e + 1]) D.pairs[to] = make_int2(ts, tss);
   }
 }
 
@@ -285,9 +287,10 @@ __global__ void __launch_bounds__(kResolveBlock) k_clean_resolve(CleanDev D) {
     atomicAdd(D.n_pairs, found);
     if (found > kMaxEventPairs) atomicOr(D.err, 2);
   }
-  const int n = min(found, D.pair_stride);
+  const long long first = D.pair_begin[e];
+  const int n = (int)min((long long)found, D.pair_begin[e + 1] - first);
   for (int p = tid; p < n; p += kResolveBlock) {
-    const int2 pr = D.pairs[(size_t)e * D.pair_stride + p];
+    const int2 pr = D.pairs[first + p];
     s_key[p] = ((long long)pr.x << 32) | (unsigned)pr.y;
     // Every seed starts as its own component.
     D.comp[pr.x] = pr.x;
@@ -413,19 +416,22 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   MKFG_REQUIRE(drmax > 0.f && drmax < 1.f, "drmax out of range");
   P.reach = (int)std::ceil(drmax * (kEtaBins / (kEtaHi - kEtaLo))) + 1;
 
-  // Pairs an event can have: what the resolve step holds, and never more
-  // than its seeds allow.
-  long long most = 1;
+  // Places for each event's pairs: what the resolve step holds, and never
+  // more than its seeds allow (at most 45 per seed, whatever the other
+  // events' sizes). The seeds' begins follow in the same array, so one copy
+  // takes both.
+  const size_t n_begin = (size_t)n_events + 1;
+  std::vector<long long> pair_begin(n_begin + (n_begin + 1) / 2, 0);
   for (int e = 0; e < n_events; ++e) {
     const long long m = event_seed_begin[e + 1] - event_seed_begin[e];
-    most = std::max(most, m * (m - 1) / 2);
+    pair_begin[e + 1] = pair_begin[e] + std::min<long long>(m * (m - 1) / 2, kMaxEventPairs);
   }
-  const int pair_stride = (int)std::min<long long>(most, kMaxEventPairs);
+  std::memcpy(&pair_begin[n_begin], event_seed_begin, 4 * n_begin);
   const int pair_cap = 8 * n + 1024;
   const size_t f_bytes = 4 * (size_t)n;
   const size_t row_bytes = 4 * (size_t)n * in_hits, out_bytes = 4 * (size_t)n * max_hits;
-  const size_t need = 6 * f_bytes * 4 + 4 * (size_t)n_events * (kEtaBins + 3) +
-                      8 * (size_t)n_events * pair_stride + 2 * row_bytes + 2 * out_bytes + 64 +
+  const size_t need = 6 * f_bytes * 4 + 4 * (size_t)n_events * (kEtaBins + 5) +
+                      8 * (size_t)pair_begin[n_events] + 2 * row_bytes + 2 * out_bytes + 64 +
                       64 * 256;
   if ((rc = ctx->scratch_misc.ensure(need))) return rc;
   char* base = ctx->scratch_misc.as<char>();
@@ -439,14 +445,14 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   D.n_events = n_events;
   D.n = n;
   D.max_hits = max_hits;
-  D.pair_stride = pair_stride;
   float* par = (float*)take(6 * f_bytes);
   int* chg = (int*)take(f_bytes);
   D.par = par;
   D.chg = chg;
-  int* evb = (int*)take(4 * (size_t)(n_events + 1));
   int* evo = (int*)take(f_bytes);
-  D.ev_begin = evb;
+  long long* begins = (long long*)take(8 * pair_begin.size());
+  D.pair_begin = begins;
+  D.ev_begin = (int*)(begins + n_begin);
   D.ev_of = evo;
   D.pt = (float*)take(f_bytes);
   D.eta = (float*)take(f_bytes);
@@ -458,7 +464,7 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   D.ebin = (int*)take(f_bytes);
   D.bin_count = (int*)take(4 * (size_t)n_events * (kEtaBins + 1));
   D.order = (int*)take(f_bytes);
-  D.pairs = (int2*)take(8 * (size_t)n_events * pair_stride);
+  D.pairs = (int2*)take(8 * (size_t)pair_begin[n_events]);
   D.comp = (int*)take(f_bytes);
   D.nh = (int*)take(f_bytes);
   D.hl = (int*)take(out_bytes);
@@ -475,7 +481,7 @@ extern "C" int mkfg_clean_seeds(mkfg_context* ctx, const mkfg_seed_clean_params*
   cudaStream_t st = ctx->stream;
   MKFG_CUDA_TRY(cudaMemcpyAsync(par, seed_par, 6 * f_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(chg, seed_chg, f_bytes, cudaMemcpyHostToDevice, st));
-  MKFG_CUDA_TRY(cudaMemcpyAsync(evb, event_seed_begin, 4 * (size_t)(n_events + 1), cudaMemcpyHostToDevice, st));
+  MKFG_CUDA_TRY(cudaMemcpyAsync(begins, pair_begin.data(), 8 * pair_begin.size(), cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(D.nh, seed_nhits, f_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(in_hl, seed_hit_layer, row_bytes, cudaMemcpyHostToDevice, st));
   MKFG_CUDA_TRY(cudaMemcpyAsync(in_hi, seed_hit_index, row_bytes, cudaMemcpyHostToDevice, st));

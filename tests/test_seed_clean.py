@@ -178,3 +178,38 @@ def test_device_components_match_restatement(gpu_ctx):
 
 def first_event(sd, n):
     return {k: (v[:, :n] if k in ("par", "err") else v[:n]) for k, v in sd.items()}
+
+
+@pytest.mark.gpu
+def test_device_scratch_follows_each_event(gpu_ctx):
+    """A large event beside 20,000 of two seeds: the scratch holds each
+    event's own pairs, not the large one's 4096 for everyone (655 MB). Needed
+    at most: the 1024-bin table of an event and, per seed, 45 pairs, the 20
+    per-seed words and the hit rows; the bound leaves twice that."""
+    import torch
+    from mkfit_b200 import Context
+    from mkfit_b200.seed_clean import clean_seeds
+    big, tiny = seeds_of(130, 41), first_event(seeds_of(130, 41), 2)
+    evs = [big] + [tiny] * 20000
+    begin = np.cumsum([0] + [len(e["chg"]) for e in evs]).astype(np.int32)
+    cat = lambda k, ax: np.concatenate([e[k] for e in evs], axis=ax)  # noqa: E731
+    args = (begin, cat("par", 1), cat("chg", 0), cat("nhits", 0), cat("hit_layer", 0),
+            cat("hit_index", 0))
+    torch.cuda.synchronize()
+    ctx = Context(0)
+    try:
+        clean_seeds(ctx, np.array([0, 2], np.int32), tiny["par"], tiny["chg"], tiny["nhits"],
+                    tiny["hit_layer"], tiny["hit_index"])
+        free = torch.cuda.mem_get_info()[0]
+        out = clean_seeds(ctx, *args)
+        used = free - torch.cuda.mem_get_info()[0]
+    finally:
+        ctx.close()
+    width = args[4].shape[1]
+    need = 20001 * 4 * 1024 + len(args[2]) * (45 * 8 + 20 * 4 + 8 * (width + 16))
+    assert used < 2 * need, (used, need)
+    # The large event as when it is cleaned alone.
+    n = begin[1]
+    alone = clean_seeds(gpu_ctx, begin[:2], *(a[:, :n] if a is args[1] else a[:n] for a in args[1:]))
+    for a, b in zip(out, alone):
+        np.testing.assert_array_equal(a[:n], b)
