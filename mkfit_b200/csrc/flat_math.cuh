@@ -1,4 +1,5 @@
-// Elementary arithmetic for the Kalman step in two forms with one result.
+// Elementary arithmetic for the Kalman step in two forms with one result but
+// for the two rare roundings named below.
 //
 // ExactMath is the plain form: IEEE division and square root, double
 // elementary functions rounded once to float (kalman.cuh f_*). Each of its
@@ -10,9 +11,10 @@
 // FlatMath computes the same values without a branch, for operands in a
 // safe range, and keeps the smallest and largest operand it was given: when
 // one lay outside (or was NaN), ok() is false and the caller repeats the step
-// with ExactMath. Methods: correctly rounded quotient and root from an
-// approximate reciprocal (root) by fused residuals (P. Markstein, IBM J. Res.
-// Dev. 34, 1990); sine and cosine by their Taylor series after reduction by
+// with ExactMath. Methods: quotient and root from an approximate reciprocal
+// (root) by fused residuals (P. Markstein, IBM J. Res. Dev. 34, 1990),
+// correctly rounded but for the reciprocal of a mantissa of all ones, which
+// is one ulp off, and quotients by such a number (two of 2^26 tried); sine and cosine by their Taylor series after reduction by
 // multiples of pi/2 in two parts; logarithm by the series of
 // 2 artanh((m - 1) / (m + 1)). The double results are within a few 1e-16 of
 // the exact value, so they round to ExactMath's float but where that value
@@ -45,8 +47,9 @@ __device__ __forceinline__ float max_nan(float a, float b) {
   return y;
 }
 
-// Correctly rounded 1 / b, a / b and sqrt(x) for operands whose size lies
-// in [2^-100, 2^100] (and a = 0).
+// 1 / b, a / b and sqrt(x) for normal operands (a may be 0) whose result is a
+// normal finite number; an overflow gives NaN. ok() leaves the step's
+// divisors and roots within [2^-80, 2^120].
 __device__ __forceinline__ float flat_rcp(float b) {
   float y = rcp_approx(b);
   y = __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
@@ -148,6 +151,9 @@ struct FlatMath {
     wlo = min_nan(wlo, v);
     whi = max_nan(whi, v);
   }
+  // A dividend, or another number that only its size can spoil: a quotient
+  // that overflows is NaN here and infinite there.
+  __device__ __forceinline__ void see_top(float v) { hi = max_nan(hi, fabsf(v)); }
   __device__ __forceinline__ void see_angle(float v) { hi = max_nan(hi, fabsf(v) * 0x1p12f); }
   __device__ __forceinline__ bool ok() const {
     return lo >= 0x1p-20f && hi <= 0x1p20f && wlo >= 0x1p-90f && whi <= 0x1p90f;

@@ -120,6 +120,7 @@ struct ExactMath {
   static constexpr bool kPlain = true;
   __device__ __forceinline__ void see(float) {}
   __device__ __forceinline__ void see_wide(float) {}
+  __device__ __forceinline__ void see_top(float) {}
   __device__ __forceinline__ bool ok() const { return true; }
   __device__ __forceinline__ static float rcp(float b) { return 1.f / b; }
   __device__ __forceinline__ static float div(float a, float b) { return a / b; }
@@ -425,6 +426,7 @@ __device__ __forceinline__ void material_effects(F& m, float radL, float xi, flo
   const float dEdx =
       beta < 1.f ? (2.f * (F::div(xi * invCos * (fmaf(0.5f, log_w, -beta2) - deltahalf), beta2))) : 0.f;
   const float dP = F::div(prop_sign * dEdx, beta);
+  m.see_top(dP);
   par[3] = F::div(p, fmaxf(p + dP, 0.001f) * pt);
   C[9] += F::div(dP * dP, p2 * pt * pt);  // (3,3)
 }
@@ -611,8 +613,11 @@ __device__ __forceinline__ float kalman_barrel_in(F& m, const float (&par)[6], c
                                                   const float (&mpos)[3], const float (&merr)[6],
                                                   float (&opar)[6], float (&oerr)[21]) {
   const float r = m.hypot(mpos[0], mpos[1]);
-  const float r00 = F::div(-(mpos[1] + par[1]), 2 * r);
-  const float r01 = F::div(mpos[0] + par[0], 2 * r);
+  const float sx = mpos[0] + par[0], sy = mpos[1] + par[1];
+  m.see_top(sx);
+  m.see_top(sy);
+  const float r00 = F::div(-sy, 2 * r);
+  const float r01 = F::div(sx, 2 * r);
 
   const float res0 = mpos[0] - par[0], res1 = mpos[1] - par[1], res2 = mpos[2] - par[2];
   // Covariance sum in global position coordinates (upper-left 3x3).

@@ -1,5 +1,6 @@
-// Compares the branch-free arithmetic of csrc/flat_math.cuh with the plain
-// one on the device; built and loaded by test_flat_math_gpu.py.
+// Compares the branch-free arithmetic of csrc/flat_math.cuh, and the steps of
+// the fit that use it, with the plain ones on the device; built and loaded by
+// test_flat_math_gpu.py.
 #include "../mkfit_b200/csrc/kalman.cuh"
 
 using namespace mkfg;
@@ -56,5 +57,74 @@ __global__ void k_seen(int n, const float* v, int wide, int* ok) {
 }
 extern "C" int flat_math_seen(int n, const float* v, int wide, int* ok) {
   k_seen<<<(n + 127) / 128, 128>>>(n, v, wide, ok);
+  return (int)cudaDeviceSynchronize();
+}
+
+// A propagation (barrel: to the hit's radius, else to its z) and an update of
+// the given state, flat and plain: out[2][55][n] (6 + 21 propagated, 6 + 21
+// updated, chi2), back[2][n]: whether the flat form would use the plain one.
+struct StepArgs {
+  int n, barrel;
+  unsigned pflags;
+  Material mat;
+  const float *par, *err, *hpos, *herr;
+  const int* chg;
+  float* out;
+  int* back;
+};
+template <bool kBarrel>
+__device__ void step_check(const StepArgs& a, int i) {
+  float p[6], e[21], m[3], v[6];
+  for (int k = 0; k < 6; ++k) p[k] = a.par[k * a.n + i];
+  for (int k = 0; k < 21; ++k) e[k] = a.err[k * a.n + i];
+  for (int k = 0; k < 3; ++k) m[k] = a.hpos[k * a.n + i];
+  for (int k = 0; k < 6; ++k) v[k] = a.herr[k * a.n + i];
+  const int chg = a.chg[i];
+  const float r = hypot_f(m[0], m[1]);
+  for (int form = 0; form < 2; ++form) {
+    float pp[6], pe[21], up[6], ue[21], chi2;
+    if (form == 0) {
+      if (kBarrel) propagate_to_r_flat(p, e, chg, r, a.pflags, a.mat, false, pp, pe);
+      else propagate_to_z_flat(p, e, chg, m[2], a.pflags, a.mat, false, pp, pe);
+    } else {
+      if (kBarrel) propagate_to_r(p, e, chg, r, a.pflags, a.mat, false, pp, pe);
+      else propagate_to_z(p, e, chg, m[2], a.pflags, a.mat, false, pp, pe);
+    }
+    // The update from the given state, which may lie anywhere.
+    if (form == 0)
+      chi2 = update_flat<true, kBarrel>(p, e, m, v, up, ue);
+    else
+      chi2 = kBarrel ? kalman_barrel<true, true>(p, e, m, v, up, ue)
+                     : kalman_endcap<true, true>(p, e, m, v, up, ue);
+    float* o = a.out + (size_t)form * 55 * a.n + i;
+    for (int k = 0; k < 6; ++k) o[k * a.n] = pp[k];
+    for (int k = 0; k < 21; ++k) o[(6 + k) * a.n] = pe[k];
+    for (int k = 0; k < 6; ++k) o[(27 + k) * a.n] = up[k];
+    for (int k = 0; k < 21; ++k) o[(33 + k) * a.n] = ue[k];
+    o[54 * a.n] = chi2;
+  }
+  FlatMath fp, fu;
+  float pp[6], pe[21];
+  if (kBarrel) {
+    propagate_to_r_in(fp, p, e, chg, r, a.pflags, a.mat, false, pp, pe);
+    kalman_barrel_in<true, true>(fu, p, e, m, v, pp, pe);
+  } else {
+    propagate_to_z_in(fp, p, e, chg, m[2], a.pflags, a.mat, false, pp, pe);
+    kalman_endcap_in<true, true>(fu, p, e, m, v, pp, pe);
+  }
+  a.back[i] = !fp.ok();
+  a.back[a.n + i] = !fu.ok();
+}
+__global__ void __launch_bounds__(128) k_step(const StepArgs a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  if (a.barrel) step_check<true>(a, i);
+  else step_check<false>(a, i);
+}
+extern "C" int flat_math_step(int n, int barrel, unsigned pflags, const float* rl, const float* xi,
+                              const float* par, const float* err, const int* chg, const float* hpos,
+                              const float* herr, float* out, int* back) {
+  const StepArgs a{n, barrel, pflags, Material{rl, xi}, par, err, hpos, herr, chg, out, back};
+  k_step<<<(n + 127) / 128, 128>>>(a);
   return (int)cudaDeviceSynchronize();
 }

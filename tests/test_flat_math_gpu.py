@@ -1,8 +1,8 @@
 """The branch-free arithmetic of the Kalman step (csrc/flat_math.cuh) against
 the plain one on the device: the quotient, reciprocal and root bit for bit
 (every mantissa for the one-operand ones), the double-based functions up to
-the values within ~1e-16 of a rounding boundary, and the operands that send a
-step back to the plain form."""
+the values within ~1e-16 of a rounding boundary, the operands that send a
+step back to the plain form, and whole steps from such states."""
 import ctypes
 import os
 import subprocess
@@ -20,12 +20,13 @@ def lib(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("flat") / "libflat.so")
     subprocess.check_call([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode",
                            "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared",
-                           "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+                           "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-fmad=false",
                            os.path.join(HERE, "flat_math_check.cu"), "-o", out])
     L = ctypes.CDLL(out)
     p = ctypes.c_void_p
     L.flat_math_check.argtypes = [ctypes.c_int, ctypes.c_longlong, p, p, p]
     L.flat_math_seen.argtypes = [ctypes.c_int, p, ctypes.c_int, p]
+    L.flat_math_step.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint] + [p] * 9
     return L
 
 
@@ -95,3 +96,66 @@ def test_operands_outside_the_range(lib):
         torch.cuda.synchronize()
         assert lib.flat_math_seen(len(v), v.data_ptr(), wide, ok.data_ptr()) == 0
         assert ok.cpu().tolist() == exp
+
+
+def step_states(barrel):
+    """Toy tracks of one layer with every special value in every place it can
+    take: parameters, covariance, charge and hit."""
+    from mkfit_b200 import synth
+    n = 40000
+    gen = synth.gen_fit_event if barrel else synth.gen_fit_event_steered
+    ev, layer = gen(n, seed=3), 3 if barrel else 2
+    rng = np.random.default_rng(7)
+    a = rng.normal(0, 1, (n, 6, 6)) * np.array([.01, .01, .05, .02, .002, .002])[None, :, None]
+    d = dict(par=ev.par.copy(), err=synth.pack_sym(a @ a.transpose(0, 2, 1)).astype(np.float32),
+             chg=ev.chg.copy(), hpos=ev.hit_pos[layer].copy(), herr=ev.hit_err[layer].copy())
+    special = np.array([0.0, -0.0, 1e-40, 1e-30, 1e-8, -1.0, 1500.0, 1e7, 3e19, -1e30, 3e38,
+                        np.inf, -np.inf, np.nan, np.pi / 2, np.pi], np.float32)
+    i = 1000  # the first 1000 stay ordinary
+    for name in ("par", "err", "hpos", "herr"):
+        for row in d[name]:
+            row[i:i + len(special)] = special
+            i += len(special)
+    for rows in (d["par"][:2], d["hpos"][:2], d["hpos"], d["err"], d["herr"]):
+        for s in special:  # at the beam line, or the whole block special
+            rows[:, i] = s
+            i += 1
+    for q in (0, 2, -3, 127):
+        d["chg"][i] = q
+        i += 1
+    assert i < n
+    return ev, {k: np.ascontiguousarray(v) for k, v in d.items()}, i
+
+
+@pytest.mark.parametrize("barrel", [1, 0])
+@pytest.mark.parametrize("grid", ["usual", "inf", "huge", "nan"])
+def test_steps_from_any_state(lib, barrel, grid):
+    """The fit's flat propagation and update equal the plain ones bit for bit,
+    infinities and NaNs included, whether or not they go back to them. The
+    double functions' results may round otherwise for about 1e-7 of the
+    values (test_functions), 6 per step: at most 2 of these tracks."""
+    import torch
+    ev, d, n_special = step_states(barrel)
+    n = len(d["chg"])
+    rl, xi = np.array(ev.rl_grid), np.array(ev.xi_grid)
+    if grid != "usual":
+        v = np.float32(dict(inf=np.inf, huge=1e38, nan=np.nan)[grid])
+        xi[::2] = v
+        rl[1::4] = v
+    t = {k: torch.from_numpy(v).cuda() for k, v in dict(d, rl=rl, xi=xi).items()}
+    for pflags in range(4):
+        out = torch.zeros((2, 55, n), device="cuda")
+        back = torch.zeros((2, n), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        assert lib.flat_math_step(n, barrel, pflags, *(t[k].data_ptr() for k in (
+            "rl", "xi", "par", "err", "chg", "hpos", "herr")), out.data_ptr(), back.data_ptr()) == 0
+        flat, plain = out.cpu().numpy()
+        bad = ((flat != plain) & ~(np.isnan(flat) & np.isnan(plain))).any(0)
+        print(f"pflags {pflags}: {bad.sum()} of {n} tracks differ, back {back.sum(1).tolist()}")
+        assert not (np.isnan(flat) != np.isnan(plain)).any()
+        assert bad.sum() <= 2, np.flatnonzero(bad)[:20]
+        # Both ways were taken: special states went back, ordinary ones did not.
+        b = back.cpu().numpy()
+        assert (b[:, 1000:n_special].sum(1) > 20).all()
+        if grid == "usual":
+            assert b[:, :1000].sum() == 0
