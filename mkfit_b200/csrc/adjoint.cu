@@ -17,87 +17,9 @@
 // the state to the previous step; per-step parameter adjoints are reduced
 // over the block in shared memory (double) and added to the global gradient.
 #include "internal.h"
-#include "kalman.cuh"
-#include "adjoint_step.cuh"
-
-#include <type_traits>
+#include "adjoint_flat.cuh"
 
 namespace mkfg {
-namespace adj {
-
-// The material grid with the branch-free quotient and root (flat_math.cuh)
-// and the range of the operands they were given.
-struct FlatGrid : MatGrid {
-  mutable float lo = 1.f, hi = 1.f;
-  __device__ __forceinline__ explicit FlatGrid(const MatGrid& g) : MatGrid(g) {}
-  __device__ __forceinline__ bool ok() const { return lo >= 0x1p-90f && hi <= 0x1p90f; }
-};
-__device__ __forceinline__ float ad_div(const FlatGrid&, float a, float b) {
-  return flat_div_y(a, b, flat_rcp(b));
-}
-__device__ __forceinline__ float ad_sqrt(const FlatGrid&, float x) { return flat_sqrt(x); }
-__device__ __forceinline__ void ad_see(const FlatGrid& m, float v) {
-  m.lo = min_nan(m.lo, fabsf(v));
-  m.hi = max_nan(m.hi, fabsf(v));
-}
-
-// The plain forms under the same interface.
-struct PlainGrid : MatGrid {
-  __device__ __forceinline__ explicit PlainGrid(const MatGrid& g) : MatGrid(g) {}
-  __device__ __forceinline__ bool ok() const { return true; }
-};
-
-// The step and its reverse with the plain forms, where an operand left the
-// range: not inlined, on copies, so the usual path keeps its registers.
-struct StepIn {
-  float par[6], err[21], m[3], me[6], ta, tb, tc, k;
-};
-struct StepState {
-  float par[6], err[21], c2;
-};
-struct StepBars {
-  float par[6], err[21], ga, gb, gc;
-};
-template <bool kMat>
-__device__ __noinline__ void step_fwd_plain(const StepIn* x, MatGrid mat, StepState* o) {
-  if (kMat)
-    barrel_step_fwd_mat(x->par, x->err, x->m, x->me, x->ta, x->tb, x->tc, x->k, mat, o->par, o->err,
-                        o->c2);
-  else
-    barrel_step_fwd_nomat(x->par, x->err, x->m, x->me, x->ta, x->tb, x->tc, x->k, mat, o->par,
-                          o->err, o->c2);
-}
-template <bool kMat>
-__device__ __noinline__ void step_rev_plain(const StepIn* x, MatGrid mat, float g, StepBars* b) {
-  StepBars o;
-  if (kMat)
-    barrel_step_rev_mat(x->par, x->err, x->m, x->me, x->ta, x->tb, x->tc, x->k, mat, b->par, b->err,
-                        g, o.par, o.err, o.ga, o.gb, o.gc);
-  else
-    barrel_step_rev_nomat(x->par, x->err, x->m, x->me, x->ta, x->tb, x->tc, x->k, mat, b->par,
-                          b->err, g, o.par, o.err, o.ga, o.gb, o.gc);
-  *b = o;
-}
-__device__ __forceinline__ StepIn step_in(const float (&par)[6], const float (&err)[21],
-                                          const float (&m)[3], const float (&me)[6], float ta,
-                                          float tb, float tc, float k) {
-  StepIn x;
-#pragma unroll
-  for (int e = 0; e < 6; ++e) x.par[e] = par[e];
-#pragma unroll
-  for (int e = 0; e < 21; ++e) x.err[e] = err[e];
-#pragma unroll
-  for (int e = 0; e < 3; ++e) x.m[e] = m[e];
-#pragma unroll
-  for (int e = 0; e < 6; ++e) x.me[e] = me[e];
-  x.ta = ta;
-  x.tb = tb;
-  x.tc = tc;
-  x.k = k;
-  return x;
-}
-
-}  // namespace adj
 
 constexpr int kAdjBlock = 128;
 constexpr int kAdjMaxSteps = 64;
@@ -180,21 +102,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_align_forward(const AdjKernelArgs
       const float ta = __ldg(a.theta + 3 * s), tb = __ldg(a.theta + 3 * s + 1),
                   tc = __ldg(a.theta + 3 * s + 2);
       float opar[6], oerr[21], c2;
-      const adj::FlatGrid mat(a.mat);
-      if (kMat)
-        adj::barrel_step_fwd_mat(par, err, m, me, ta, tb, tc, k, mat, opar, oerr, c2);
-      else
-        adj::barrel_step_fwd_nomat(par, err, m, me, ta, tb, tc, k, mat, opar, oerr, c2);
-      if (!mat.ok()) {
-        const adj::StepIn x = adj::step_in(par, err, m, me, ta, tb, tc, k);
-        adj::StepState o;
-        adj::step_fwd_plain<kMat>(&x, a.mat, &o);
-#pragma unroll
-        for (int e = 0; e < 6; ++e) opar[e] = o.par[e];
-#pragma unroll
-        for (int e = 0; e < 21; ++e) oerr[e] = o.err[e];
-        c2 = o.c2;
-      }
+      adj::step_fwd<kMat>(par, err, m, me, ta, tb, tc, k, a.mat, opar, oerr, c2);
 #pragma unroll
       for (int e = 0; e < 6; ++e) par[e] = opar[e];
 #pragma unroll
@@ -252,30 +160,8 @@ __global__ void __launch_bounds__(kAdjBlock) k_align_backward(const AdjKernelArg
       const float ta = __ldg(a.theta + 3 * s), tb = __ldg(a.theta + 3 * s + 1),
                   tc = __ldg(a.theta + 3 * s + 2);
       float pb[6], eb[21];
-      using Grid = std::conditional_t<kFlat, adj::FlatGrid, adj::PlainGrid>;
-      const Grid mat(a.mat);
-      if (kMat)
-        adj::barrel_step_rev_mat(par, err, m, me, ta, tb, tc, k, mat, par_bar, err_bar, g, pb, eb,
+      adj::step_rev<kMat, kFlat>(par, err, m, me, ta, tb, tc, k, a.mat, par_bar, err_bar, g, pb, eb,
                                  ga, gb, gc);
-      else
-        adj::barrel_step_rev_nomat(par, err, m, me, ta, tb, tc, k, mat, par_bar, err_bar, g, pb, eb,
-                                   ga, gb, gc);
-      if (!mat.ok()) {
-        const adj::StepIn x = adj::step_in(par, err, m, me, ta, tb, tc, k);
-        adj::StepBars o;
-#pragma unroll
-        for (int e = 0; e < 6; ++e) o.par[e] = par_bar[e];
-#pragma unroll
-        for (int e = 0; e < 21; ++e) o.err[e] = err_bar[e];
-        adj::step_rev_plain<kMat>(&x, a.mat, g, &o);
-#pragma unroll
-        for (int e = 0; e < 6; ++e) pb[e] = o.par[e];
-#pragma unroll
-        for (int e = 0; e < 21; ++e) eb[e] = o.err[e];
-        ga = o.ga;
-        gb = o.gb;
-        gc = o.gc;
-      }
 #pragma unroll
       for (int e = 0; e < 6; ++e) par_bar[e] = pb[e];
 #pragma unroll

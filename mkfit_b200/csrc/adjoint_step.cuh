@@ -16,12 +16,14 @@ namespace mkfg {
 namespace adj {
 
 // Quotient and root, and the operands whose size they need in a safe range:
-// here the plain forms, for any material argument; adjoint.cu adds the
+// here the plain forms, for any material argument; adjoint_flat.cuh adds the
 // branch-free ones for its own.
 template <typename T, typename MatT>
 AD_FN T ad_div(const MatT&, T a, T b) { return a / b; }
 template <typename T, typename MatT>
 AD_FN void ad_see(const MatT&, T) {}
+template <typename T, typename MatT>
+AD_FN void ad_see_top(const MatT&, T) {}
 template <typename MatT>
 AD_FN float ad_sqrt(const MatT&, float x) { return sqrtf(x); }
 template <typename MatT>

@@ -472,6 +472,8 @@ class Emitter:
                     n.args[watched].id not in self.seen:
                 self.seen.add(n.args[watched].id)
                 lines.append("  ad_see(mat, %s);" % A[watched])
+            if op == "max":  # would drop a NaN
+                lines.append("  ad_see_top(mat, %s);" % A[0])
             lines.append("  const T %s = %s;" % (v, expr))
         return order
 

@@ -15,14 +15,18 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 RCP, DIV, SQRT, SIN, COS, LOG, HYPOT, INV_DET = range(8)
 
 
-@pytest.fixture(scope="module")
-def lib(tmp_path_factory):
-    out = str(tmp_path_factory.mktemp("flat") / "libflat.so")
+def built(tmp_path_factory, name):
+    out = str(tmp_path_factory.mktemp("flat") / f"lib{name}.so")
     subprocess.check_call([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode",
                            "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared",
                            "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-fmad=false",
-                           os.path.join(HERE, "flat_math_check.cu"), "-o", out])
-    L = ctypes.CDLL(out)
+                           os.path.join(HERE, name + ".cu"), "-o", out])
+    return ctypes.CDLL(out)
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    L = built(tmp_path_factory, "flat_math_check")
     p = ctypes.c_void_p
     L.flat_math_check.argtypes = [ctypes.c_int, ctypes.c_longlong, p, p, p]
     L.flat_math_seen.argtypes = [ctypes.c_int, p, ctypes.c_int, p]
@@ -159,3 +163,46 @@ def test_steps_from_any_state(lib, barrel, grid):
         assert (b[:, 1000:n_special].sum(1) > 20).all()
         if grid == "usual":
             assert b[:, :1000].sum() == 0
+
+
+@pytest.fixture(scope="module")
+def adjoint_lib(tmp_path_factory):
+    L = built(tmp_path_factory, "adjoint_flat_check")
+    L.adjoint_flat_step.argtypes = [ctypes.c_int] + [ctypes.c_void_p] * 5
+    return L
+
+
+@pytest.mark.parametrize("grid", ["usual", "inf", "huge", "nan"])
+def test_differentiable_steps_from_any_state(adjoint_lib, grid):
+    """The same for a step of the differentiable fit and its reverse, with
+    special values in the gradients that enter it too (built without
+    contraction on both sides, the only thing that may tell them apart but
+    for the reciprocals of a mantissa of all ones: at most 2 tracks)."""
+    import torch
+    ev, d, _ = step_states(1)
+    n = len(d["chg"])
+    rng = np.random.default_rng(8)
+    inp = np.concatenate([d["par"], d["err"], d["hpos"], d["herr"], np.ones((1, n), np.float32),
+                          d["chg"][None].astype(np.float32)])
+    bars = rng.normal(0, 1, (27, n)).astype(np.float32) * 10.0 ** rng.integers(-4, 5, (27, 1))
+    bars = bars.astype(np.float32)
+    special = np.array([0.0, -0.0, 1e-40, 1e-30, 1e30, 3e38, np.inf, -np.inf, np.nan], np.float32)
+    i = 2000
+    for row in [inp[36]] + list(bars):
+        row[i:i + len(special)] = special
+        i += len(special)
+    bars[:, i:i + 200] = 0
+    rl, xi = np.array(ev.rl_grid), np.array(ev.xi_grid)
+    if grid != "usual":
+        v = np.float32(dict(inf=np.inf, huge=1e38, nan=np.nan)[grid])
+        xi[::2] = v
+        rl[1::4] = v
+    t = [torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (inp, bars, rl, xi)]
+    out = torch.zeros((2, 58, n), device="cuda")
+    torch.cuda.synchronize()
+    assert adjoint_lib.adjoint_flat_step(n, *(x.data_ptr() for x in t), out.data_ptr()) == 0
+    flat, plain = out.cpu().numpy()
+    assert np.isfinite(plain[:, :1000]).all() or grid != "usual"
+    bad = ((flat != plain) & ~(np.isnan(flat) & np.isnan(plain))).any(0)
+    print(f"{bad.sum()} of {n} tracks differ; non-finite {(~np.isfinite(plain)).any(0).sum()}")
+    assert bad.sum() <= 2, (np.flatnonzero(bad)[:20], np.flatnonzero(bad).size)
