@@ -124,14 +124,15 @@ __global__ void __launch_bounds__(kAdjBlock) k_align_forward(const AdjKernelArgs
 
 // Bound by latency (255 registers, 8 warps per SM) and the spills of the
 // reverse sweep's thousand live values. The branch-free quotients and roots
-// (kFlat) shorten its chains but lengthen the live ranges: 10 steps of 3001
-// tracks 62.6 against 82.0 us with material, 55.4 against 67.7 without;
-// 37,800 tracks 104.9 against 92.4 with (so the plain form there, from where
-// a second block per SM is needed), 63.7 against 76.0 without; 50,000 without
-// 117 against 140. 168 registers (3 blocks per SM) gave 171 against 177 us at
-// 50,000 with material, but 92 against 82 at 3001. The forward kernel gains
-// at every size (24.5 against 33.0 us at 3001, 41.2 against 47.3 at 50,000).
-template <bool kMat, bool kFlat>
+// shorten its chains and lengthen the live ranges (468 against 296 bytes
+// spilled with material), which pays at every size: 10 steps with material
+// 63 against 82 us for 3001 tracks, 76 against 90 for 19,000 and for 37,800,
+// 146 against 178 for 50,000, 234 against 277 for 100,000; without material
+// 55 against 68 for 3001, 117 against 140 for 50,000. 168 registers (3 blocks
+// per SM) gave 171 us at 50,000 with material and the plain forms. The forward
+// kernel gains at every size (24 against 33 us at 3001, 41 against 47 at
+// 50,000).
+template <bool kMat>
 __global__ void __launch_bounds__(kAdjBlock) k_align_backward(const AdjKernelArgs a) {
   __shared__ double acc[kAdjMaxSteps * 3];
   for (int j = threadIdx.x; j < 3 * a.n_steps; j += blockDim.x) acc[j] = 0.0;
@@ -160,8 +161,8 @@ __global__ void __launch_bounds__(kAdjBlock) k_align_backward(const AdjKernelArg
       const float ta = __ldg(a.theta + 3 * s), tb = __ldg(a.theta + 3 * s + 1),
                   tc = __ldg(a.theta + 3 * s + 2);
       float pb[6], eb[21];
-      adj::step_rev<kMat, kFlat>(par, err, m, me, ta, tb, tc, k, a.mat, par_bar, err_bar, g, pb, eb,
-                                 ga, gb, gc);
+      adj::step_rev<kMat>(par, err, m, me, ta, tb, tc, k, a.mat, par_bar, err_bar, g, pb, eb, ga, gb,
+                          gc);
 #pragma unroll
       for (int e = 0; e < 6; ++e) par_bar[e] = pb[e];
 #pragma unroll
@@ -268,19 +269,10 @@ extern "C" int mkfg_align_chi2_backward(mkfg_context* ctx, const mkfg_align_args
   MKFG_CUDA_TRY(cudaMemsetAsync(grad_theta, 0, sizeof(double) * 3 * k.n_steps, ctx->stream));
   if (k.n == 0) return MKFG_OK;
   const int grid = (k.n + kAdjBlock - 1) / kAdjBlock;
-  // The branch-free form where a block per SM holds all tracks (material on)
-  // or always (off); see k_align_backward.
-  int n_sm = 0;
-  MKFG_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, ctx->device));
-  const bool flat = !k.material || grid <= n_sm;
-  if (k.material && flat)
-    k_align_backward<true, true><<<grid, kAdjBlock, 0, ctx->stream>>>(k);
-  else if (k.material)
-    k_align_backward<true, false><<<grid, kAdjBlock, 0, ctx->stream>>>(k);
-  else if (flat)
-    k_align_backward<false, true><<<grid, kAdjBlock, 0, ctx->stream>>>(k);
+  if (k.material)
+    k_align_backward<true><<<grid, kAdjBlock, 0, ctx->stream>>>(k);
   else
-    k_align_backward<false, false><<<grid, kAdjBlock, 0, ctx->stream>>>(k);
+    k_align_backward<false><<<grid, kAdjBlock, 0, ctx->stream>>>(k);
   MKFG_CUDA_TRY(cudaGetLastError());
   return MKFG_OK;
 }

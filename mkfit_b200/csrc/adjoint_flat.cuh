@@ -6,8 +6,6 @@
 #include "kalman.cuh"
 #include "adjoint_step.cuh"
 
-#include <type_traits>
-
 namespace mkfg {
 namespace adj {
 
@@ -35,15 +33,6 @@ __device__ __forceinline__ void ad_see_all(const FlatGrid& m, const float (&v)[N
 #pragma unroll
   for (int e = 0; e < N; ++e) ad_see_top(m, v[e]);
 }
-
-// The plain forms under the same interface.
-struct PlainGrid : MatGrid {
-  __device__ __forceinline__ explicit PlainGrid(const MatGrid& g) : MatGrid(g) {}
-  __device__ __forceinline__ bool ok() const { return true; }
-};
-__device__ __forceinline__ void ad_see_top(const PlainGrid&, float) {}
-template <int N>
-__device__ __forceinline__ void ad_see_all(const PlainGrid&, const float (&)[N]) {}
 
 // The step and its reverse with the plain forms, where an operand left the
 // range: not inlined, on copies, so the usual path keeps its registers.
@@ -119,16 +108,14 @@ __device__ __forceinline__ void step_fwd(const float (&par)[6], const float (&er
   c2 = o.c2;
 }
 
-// kFlat: with the branch-free forms.
-template <bool kMat, bool kFlat>
+template <bool kMat>
 __device__ __forceinline__ void step_rev(const float (&par)[6], const float (&err)[21],
                                          const float (&m)[3], const float (&me)[6], float ta, float tb,
                                          float tc, float k, const MatGrid& grid,
                                          const float (&par_bar)[6], const float (&err_bar)[21], float g,
                                          float (&pb)[6], float (&eb)[21], float& ga, float& gb,
                                          float& gc) {
-  using Grid = std::conditional_t<kFlat, FlatGrid, PlainGrid>;
-  const Grid mat(grid);
+  const FlatGrid mat(grid);
   if (kMat)
     barrel_step_rev_mat(par, err, m, me, ta, tb, tc, k, mat, par_bar, err_bar, g, pb, eb, ga, gb, gc);
   else

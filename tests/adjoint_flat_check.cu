@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(128) k_adj(int n, const float* in, const float
     adj::StepBars b;
     if (form == 0) {
       adj::step_fwd<true>(par, err, m, me, 0.f, 0.f, 1.f, kk, grid, o.par, o.err, o.c2);
-      adj::step_rev<true, true>(par, err, m, me, 0.f, 0.f, 1.f, kk, grid, pbar, ebar, g, b.par, b.err,
+      adj::step_rev<true>(par, err, m, me, 0.f, 0.f, 1.f, kk, grid, pbar, ebar, g, b.par, b.err,
                                 b.ga, b.gb, b.gc);
     } else {
       adj::step_fwd_plain<true>(&x, grid, &o);
