@@ -525,12 +525,19 @@ def run_fit(ctx, stream, batch, args):
             "achieved_tflops": flops / (t * 1e-3) / 1e12}
 
 
+# Why a figure of the reference CPU build is not there.
+NO_REFERENCE = ("reference CPU build oracle/_ref missing (built by __graft_entry__.build "
+                "from the reference sources)")
+
+
 def cpu_baseline_fit(batch, n_sample):
     """The reference's MkFitter fitting loop (runFittingTestPlex:
     InputTracksForFit + FitTracksWithInterSlurp + OutputFittedTracks over
     NN-track chunks, mkFit/fittestMPlex.cc:65-100) on all host threads,
     best of 3, on the first n_sample tracks of the step."""
-    from oracle.oracle import RefLib
+    from oracle.oracle import RefLib, have_ref
+    if not have_ref():
+        return {"unavailable": NO_REFERENCE}
     ref = RefLib()
     threads = os.cpu_count()
     ref.set_threads(threads)
@@ -725,7 +732,9 @@ def cpu_baseline_find(events, gpu_best=None, n_sample=None):
     in flight), best of 3, on the first n_sample events (all by default);
     with gpu_best (the GPU's best candidate per seed of the same events),
     also the best-candidate hit-list mismatch rate against the GPU."""
-    from oracle.oracle import RefLib, ref_find_batch
+    from oracle.oracle import RefLib, have_ref, ref_find_batch
+    if not have_ref():
+        return {"unavailable": NO_REFERENCE}
     ref = RefLib()
     threads = os.cpu_count()
     ref.set_threads(threads)
@@ -761,9 +770,7 @@ def run_reference(args):
         return
     from oracle.oracle import RefLib, have_ref, ref_find_batch
     if not have_ref():
-        emit({"impl": "reference", "unavailable":
-              "reference CPU build oracle/_ref missing (built by __graft_entry__.build "
-              "from the reference sources)"})
+        emit({"impl": "reference", "unavailable": NO_REFERENCE})
         return
     events = generate(find_event_args(args.events, 0))
     ref = RefLib()

@@ -48,3 +48,20 @@ def test_reference_arm_under_two_ranks(reflib):
     d = json.loads(lines[0])
     assert d["impl"] == "reference" and d["n_gpus"] == 2
     assert d["config"]["parallelism"].startswith("dp2")
+
+
+def test_lines_without_the_reference_build(monkeypatch, capsys):
+    """Where the reference sources were not there to be built, both arms still
+    print their line: the GPU arm's CPU figures say why they are absent."""
+    import argparse
+
+    import bench
+    import oracle.oracle
+    monkeypatch.setattr(oracle.oracle, "have_ref", lambda flavour="avx2": False)
+    for k in ("RANK", "WORLD_SIZE"):
+        monkeypatch.delenv(k, raising=False)
+    assert bench.cpu_baseline_fit(None, 8) == {"unavailable": bench.NO_REFERENCE}
+    assert bench.cpu_baseline_find([]) == {"unavailable": bench.NO_REFERENCE}
+    bench.run_reference(argparse.Namespace(events=2, steps=1, warmup=1))
+    assert json.loads(capsys.readouterr().out) == {"impl": "reference",
+                                                   "unavailable": bench.NO_REFERENCE}
