@@ -424,7 +424,11 @@ int mkfg_find_run(mkfg_context* ctx);
 /* The same sequence captured once per upload into a CUDA graph and
  * replayed (one graph launch per call). Uploads of up to 7168 seeds run
  * through the fused form (mkfg_find_run_fused) instead, which is faster
- * there; so does mkfg_find_event. No reference counterpart. */
+ * there; so does mkfg_find_event. The results are the same bit for bit; the
+ * launch configuration and bin staging (mkfg_find_set_graph_tuning,
+ * mkfg_find_autotune_graph, mkfg_find_set_bin_staging) concern the launch
+ * sequence, so they do not reach such an upload's run. No reference
+ * counterpart. */
 int mkfg_find_run_graph(mkfg_context* ctx);
 /* The plain run with a CUDA event after every launch: kernel_ms[7]
  * receives the device time of each kernel class summed over the layer
@@ -434,7 +438,7 @@ int mkfg_find_run_timed(mkfg_context* ctx, float* kernel_ms);
 /* Per layer-plan step of the last run: launch_ms[max_steps][5] the device
  * time of each step launch of the last mkfg_find_run_timed (activate,
  * propagate, chi2, clone, update), counts[max_steps][7] the work of the
- * last run of any form that fills them (plain, graph, timed): active
+ * last run of any form (plain, graph, timed, fused): active
  * candidates in barrel / endcap layers, (candidate, hit) pairs barrel /
  * endcap, Kalman updates barrel / endcap, seeds finding. Either pointer may
  * be null. No reference counterpart (diagnostics). */
@@ -742,7 +746,8 @@ int mkfg_find_set_arena_capacity(mkfg_context* ctx, int32_t nodes_per_seed);
  * one of its event's hits. */
 int mkfg_find_set_seed_import(mkfg_context* ctx, int32_t on_host);
 
-/* on = 1: the propagation kernel of the following runs copies, per chunk
+/* on = 1: the propagation kernel of the following runs of the launch
+ * sequence (the fused form has none) copies, per chunk
  * of 256 active candidates, the (q bin, phi bin) table of the chunk's
  * first (event, layer) into shared memory with one bulk copy (TMA,
  * cp.async.bulk + mbarrier) and scans it there; 0 (the default): every
@@ -756,8 +761,9 @@ int mkfg_find_set_bin_staging(mkfg_context* ctx, int32_t on);
  * the propagation, chi2, clone and update kernels as a multiple of the
  * blocks the device keeps resident for each (grid_mult[4]), and the bin
  * staging of mkfg_find_set_bin_staging. ms_before / ms_after: the step
- * time (sum of the per-launch device times of one run) before and after
- * a tuning. No reference counterpart. */
+ * time (sum of the per-launch device times of one run of the launch
+ * sequence, as mkfg_find_run_timed) before and after a tuning. No reference
+ * counterpart. */
 typedef struct {
   int32_t grid_mult[4];
   int32_t stage_bins;
@@ -765,7 +771,9 @@ typedef struct {
   float ms_after;
 } mkfg_graph_tuning;
 
-/* Tunes the launch configuration on the uploaded batch: each kernel's
+/* Tunes the launch configuration on the uploaded batch (for runs of the
+ * launch sequence: mkfg_find_run, and mkfg_find_run_graph on more than 7168
+ * seeds): each kernel's
  * grid multiple in turn over 1 .. 16 by its own device time (each setting
  * timed `reps` times, the minimum kept), then the bin staging by the
  * propagation kernel's time; the choice stays with the context for its
@@ -780,7 +788,8 @@ int mkfg_find_get_graph_tuning(mkfg_context* ctx, mkfg_graph_tuning* t);
 /* Clone-step counters of the last mkfg_find_work call: the records
  * (IdxChi2List entries, hits and holes) present when the seeds were ranked
  * and the new candidates written. Counted by the eager run (mkfg_find_run)
- * only; zero after a graph replay. Diagnostic; no reference counterpart
+ * and the fused form; zero after a graph replay. Diagnostic; no reference
+ * counterpart
  * (the reference's CandCloner keeps no such totals). */
 int mkfg_find_work_clone(mkfg_context* ctx, int64_t* records, int64_t* new_cands);
 int mkfg_find_download(mkfg_context* ctx, int32_t n_seeds, mkfg_find_out* out);

@@ -2131,14 +2131,17 @@ static int enqueue_fused(Finder* f, cudaStream_t st, int w) {
 
 // Seeds per block with which a run of S seeds goes through the fused form
 // instead of the launch sequence, 0 for the sequence. A sequence of 211
-// launches costs their latency whatever the size (1.45 ms for one event of
-// 120 seeds as a graph, 1.88 ms launch by launch), and the fused form's
-// blocks run through all steps on their own: while they fit the chip at
-// once it takes 0.78 (120 seeds), 0.75 (800) and 0.87 ms (1600) with 8 seeds
-// per block, as against 0.85 with 16 per block there, which are the faster
-// ones beyond (0.95 against 1.39 ms at 3000 seeds, the graph 1.72; 1.93 at
-// 8000, the graph 2.09). The lines: where the two widths cross, and a wave of the
-// 128-thread blocks (three per SM) before the graph is the faster one.
+// launches costs their latency whatever the size (1.6 ms for one event of
+// 120 seeds as a graph, 1.9 launch by launch), and the fused form's blocks
+// run through all steps on their own. Fused against graph, ms: 120 seeds 0.78
+// / 1.59, 800 0.73 / 1.67, 1600 0.80 / 1.75, 3000 0.94 / 1.80, 5000 1.4 /
+// 2.0; from a pileup event (10,000 tracks, twice as many noise hits) 800
+// seeds 1.2 / 2.1, 3000 1.4 / 2.3, 7000 2.4 / 2.6; iterations 4 and 9 within
+// 5% of these, 7 with its short plan 0.07 / 0.25. They cross between 8200
+// seeds (1.80 / 2.01, pileup 2.21 / 2.45) and 9000 (2.13 / 2.05, 2.66 /
+// 2.55), whatever the noise: the upper line keeps clear of it. The lower one
+// is where the two widths cross (8 per block 0.73, 16 0.83 at 800 seeds; 0.86
+// and 0.81 at 1600).
 static int fused_width(int S) { return S <= 1536 ? 8 : S <= 7168 ? 16 : 0; }
 
 // The plain sequence with an event after every launch: device time per

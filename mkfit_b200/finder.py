@@ -537,9 +537,10 @@ class Finder:
         return o
 
     def autotune_graph(self, reps=2):
-        """Tunes the graph form's launch configuration on the uploaded
-        batch (mkfg_find_autotune_graph); returns it as a dict with the
-        step time before and after."""
+        """Tunes the launch sequence's configuration on the uploaded batch
+        (mkfg_find_autotune_graph; run_graph takes the fused form instead
+        up to 7168 seeds); returns it as a dict with the sequence's time
+        before and after."""
         t = MkfgGraphTuning()
         capi.check(self.lib.mkfg_find_autotune_graph(self.ctx.handle, int(reps), ctypes.byref(t)))
         return dict(grid_mult=list(t.grid_mult), stage_bins=int(t.stage_bins),

@@ -296,14 +296,26 @@ def test_find_no_seeds(gpu_ctx):
     assert out["n_cands"].shape == (0,)
 
 
+# Uploads of up to this many seeds run through the fused form in run_graph and
+# find_event (find.cu, fused_width): a test of the graph uploads more.
+FUSED_SEEDS = 7168
+
+
+def launch_sequence(fnd, ev):
+    fnd.upload(ev)
+    fnd.run()
+    return fnd.download(ev.n_seeds)
+
+
 def test_batched_graph_equals_plain(gpu_ctx):
     """The batched form (several uneven events uploaded together, found by
     one CUDA-graph replay) returns, seed for seed, the plain form's results;
     replaying the graph is repeatable."""
-    events = [synth.gen_cms_event(n, seed=100 + n, noise_frac=0.02) for n in (150, 600, 37)]
+    events = [synth.gen_cms_event(n, seed=100 + n, noise_frac=0.02) for n in (150, 6800, 600, 37)]
     fnd = Finder(gpu_ctx, FindConfig(max_cands=M))
-    plain = [fnd.find_event(ev) for ev in events]
+    plain = [launch_sequence(fnd, ev) for ev in events]
     total = fnd.upload_batch(events)
+    assert total > FUSED_SEEDS
     fnd.run_graph()
     a = fnd.download(total)
     fnd.run_graph()
@@ -315,8 +327,9 @@ def test_batched_graph_equals_plain(gpu_ctx):
         n = ev.n_seeds
         for k in ("n_cands", "region"):
             np.testing.assert_array_equal(a[k][off:off + n], p[k], err_msg=k)
-        for k in ("par", "err", "chi2", "score", "nfound", "ntot", "hit_idx", "hit_lyr"):
-            np.testing.assert_array_equal(a[k][off * M:(off + n) * M], p[k], err_msg=k)
+        for k in p:
+            if k not in ("n_cands", "region"):
+                np.testing.assert_array_equal(a[k][off * M:(off + n) * M], p[k], err_msg=k)
         off += n
     w = fnd.work()
     assert w["active_cands"] > 0 and w["hit_pairs"] > 0 and w["updates"] > 0
@@ -380,9 +393,10 @@ def test_small_uploads_equal_plain(gpu_ctx, sizes, it):
 
 
 def test_fused_autotune_and_repeat(gpu_ctx):
-    events = [synth.gen_cms_event(n, seed=300 + n) for n in (800, 300)]
+    events = [synth.gen_cms_event(n, seed=300 + n) for n in (800, 300, 6700)]
     fnd = Finder(gpu_ctx, FindConfig(max_cands=M))
     total = fnd.upload_batch(events)
+    assert total > FUSED_SEEDS
     w, ms = fnd.autotune()
     assert w in (4, 8, 16) and ms > 0
     a = fnd.download(total)
@@ -392,7 +406,6 @@ def test_fused_autotune_and_repeat(gpu_ctx):
     c = fnd.download(total)
     for k in a:
         np.testing.assert_array_equal(a[k], b[k], err_msg=k)
-    for k in ("n_cands", "hit_idx", "hit_lyr", "ntot"):
         np.testing.assert_array_equal(a[k], c[k], err_msg=k)
 
 
@@ -448,7 +461,7 @@ def test_backward_fit_matches_reference(gpu_ctx, reflib, restate, n_tracks, seed
 
 
 def test_backward_fit_batched_equals_plain(gpu_ctx):
-    events = [synth.gen_cms_event(n, seed=400 + n, noise_frac=0.02) for n in (300, 41)]
+    events = [synth.gen_cms_event(n, seed=400 + n, noise_frac=0.02) for n in (300, 7000, 41)]
     fnd = Finder(gpu_ctx, FindConfig(max_cands=M))
     plain = []
     for ev in events:
@@ -457,6 +470,7 @@ def test_backward_fit_batched_equals_plain(gpu_ctx):
         fnd.backward_fit()
         plain.append(fnd.download(ev.n_seeds))
     total = fnd.upload_batch(events)
+    assert total > FUSED_SEEDS
     fnd.run_graph()
     fnd.backward_fit()
     a = fnd.download(total)
@@ -604,7 +618,7 @@ def test_backward_search_matches_reference(gpu_ctx, reflib, n_tracks, seed, nois
 
 
 def test_backward_search_batched_equals_plain(gpu_ctx):
-    events = [synth.gen_cms_event(n, seed=500 + n, noise_frac=0.02) for n in (300, 57)]
+    events = [synth.gen_cms_event(n, seed=500 + n, noise_frac=0.02) for n in (300, 7000, 57)]
     fnd = Finder(gpu_ctx, FindConfig(max_cands=M))
     plain = []
     for ev in events:
@@ -614,6 +628,7 @@ def test_backward_search_batched_equals_plain(gpu_ctx):
         fnd.backward_search()
         plain.append(fnd.download(ev.n_seeds))
     total = fnd.upload_batch(events)
+    assert total > FUSED_SEEDS
     fnd.run_graph()
     fnd.backward_fit()
     fnd.backward_search()
