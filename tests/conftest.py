@@ -13,6 +13,15 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: longer CPU test")
 
 
+def pytest_collection_modifyitems(items):
+    """Without the reference build its tests fail, as they must; they come
+    after the others then, so that a run that stops at the first failure has
+    seen those."""
+    from oracle.oracle import have_ref
+    if not have_ref():
+        items.sort(key=lambda item: "reflib" in item.fixturenames)
+
+
 @pytest.fixture(scope="session")
 def reflib():
     from oracle.oracle import RefLib, have_ref
